@@ -1,7 +1,7 @@
 """ORDER BY of GROUP BY results on the GPU (qdb_order_by_column / qdb_order_by / qdb_reorder, the replacement of
 GPUOrderBy, qikkDB/QueryEngine/GPUCore/GPUOrderBy.cuh:88-195) against the oracle: the reference's GROUP BY +
 ORDER BY known answers, then random multi-column orders with NULLs, ties, descending columns, IEEE edge values and
-row counts around the 2048-row tile, OFFSET / LIMIT through the gather, and an ORDER BY of the 16.8M-group result
+row counts around a tile, OFFSET / LIMIT through the gather, and an ORDER BY of the 16.8M-group result
 of the composite-key GROUP BY.  Permutations must equal the oracle's exactly (the sort is stable)."""
 import json
 import os
@@ -104,3 +104,33 @@ def test_order_by_composite_groupby_results(cuda):
     idx = order_by([s, k0, k1], [True, False, False]).cpu().numpy()
     exp = oracle.order_by([s.cpu().numpy(), k0.cpu().numpy(), k1.cpu().numpy()], [True, False, False])
     assert g > 10_000_000 and (idx == exp).all()
+
+
+@pytest.mark.parametrize("n", [1, 31, 255, 257, 4095, 4096, 4097, 6144, 8191, 8192, 8193, 12_289, 300_007])
+@pytest.mark.parametrize("shape", ["constant", "one_digit", "wide", "columns"])
+def test_order_by_forms_and_skipped_digits(cuda, n, shape):
+    """Both forms of the sort (one block up to 8192 rows, tiles of 4096 64-bit or 6144 32-bit keys above) at the edges
+    of their tiles, with digits that are the same in every row (passes that do not run, in any place of the order,
+    or all of them) and more columns than one launch of the one-block form takes."""
+    rng = np.random.default_rng(n)
+    nulls = None
+    if shape == "constant":
+        cols = [np.full(n, 7, np.int64), np.full(n, -3, np.int32)]
+    elif shape == "one_digit":
+        cols = [(rng.integers(0, 256, n).astype(np.int64) << 40) + 5, (rng.integers(0, 3, n) << 8).astype(np.int32)]
+    elif shape == "wide":
+        cols = [rng.integers(-(1 << 62), 1 << 62, n), rng.standard_normal(n).astype(np.float32)]
+        nulls = [pack_nullmask(rng.random(n) < 0.3), None]
+    else:
+        cols = [rng.integers(0, 2, n).astype(np.int32 if i % 2 else np.float64) for i in range(11)]
+    desc = [bool(i % 2) for i in range(len(cols))]
+    exp = oracle.order_by(cols, desc, nulls if nulls else [None] * len(cols))
+    got = order_by([_dev(c) for c in cols], desc,
+                   [None if x is None else _dev(x.view(np.int64)) for x in nulls] if nulls else None).cpu().numpy()
+    assert (got == exp).all()
+    # the same, column by column (the permutation is read back in)
+    ob = GPUOrderBy(n)
+    for i in reversed(range(len(cols))):
+        ob.OrderByColumn(None, _dev(cols[i]), None if not nulls or nulls[i] is None else _dev(nulls[i].view(np.int64)),
+                         n, int(desc[i]))
+    assert (ob.indices[:n].cpu().numpy() == exp).all()
