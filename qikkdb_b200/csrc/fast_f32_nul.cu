@@ -1,0 +1,8 @@
+// Fast aggregation pass of calls with NULL masks or a row mask, float keys (groupby_fast.cuh).
+#include "groupby_fast.cuh"
+
+namespace qdb {
+int32_t launch_fast_f32_nul(const AggArgs& a, ValKind vk, size_t smem, cudaStream_t st) {
+    return launch_fast_nul_k<float>(a, vk, smem, st);
+}
+}  // namespace qdb

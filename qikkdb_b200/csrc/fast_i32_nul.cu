@@ -1,0 +1,8 @@
+// Fast aggregation pass of calls with NULL masks or a row mask, int32_t keys (groupby_fast.cuh).
+#include "groupby_fast.cuh"
+
+namespace qdb {
+int32_t launch_fast_i32_nul(const AggArgs& a, ValKind vk, size_t smem, cudaStream_t st) {
+    return launch_fast_nul_k<int32_t>(a, vk, smem, st);
+}
+}  // namespace qdb

@@ -100,6 +100,14 @@ static int32_t launch_spill(const qdb_gb* gb, const AggArgs& a, size_t smem, int
 
 static int32_t launch_fast(const qdb_gb* gb, const AggArgs& a, int32_t ptype, size_t smem, cudaStream_t st) {
     const ValKind vk = val_kind(gb->val_type);
+    if (a.nul) {
+        switch (gb->key_type) {
+            case QDB_INT32: return launch_fast_i32_nul(a, vk, smem, st);
+            case QDB_INT64: return launch_fast_i64_nul(a, vk, smem, st);
+            case QDB_FLOAT: return launch_fast_f32_nul(a, vk, smem, st);
+            default: return launch_fast_f64_nul(a, vk, smem, st);
+        }
+    }
     if (a.kmod) {
         if (gb->n_key_cols == 1 && gb->key_type == QDB_INT32) return launch_fast_i32_mod(a, vk, ptype, smem, st);
         if (gb->n_key_cols == 1 && gb->key_type == QDB_INT64) return launch_fast_i64_mod(a, vk, ptype, smem, st);
@@ -334,6 +342,8 @@ PredInterval pred_interval(const qdb_pred& p) {
 // columns are 16-byte aligned and hold at least one whole tile.  *used is false when the plan does not fit shared
 // memory (the caller then takes the general pass).
 // ---------------------------------------------------------------------------------------------
+constexpr size_t kMaxStates = 8192;  // states of a table with copies (clearing and merging them stays a few us)
+
 static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t ptype, cudaStream_t s, bool* used) {
     *used = false;
     const DeviceInfo& di = device_info();
@@ -343,10 +353,17 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
     const int ks = (gb->n_key_cols == 2) ? 4 : type_size(gb->key_type);
     const int vs = a.vals ? type_size(gb->val_type) : 0;
     const int ps = a.pcol ? type_size(pred->type) : 0;
-    const int row_bytes = ks * gb->n_key_cols + vs + ps;
+    const int ms = a.mask ? 1 : 0;
+    const int row_bytes = ks * gb->n_key_cols + vs + ps + ms;
+    if (a.nul) {
+        a.ptype = ptype;
+        a.null_keys = a.knull0 != nullptr;
+        a.wide = vk == VK_F64 && a.has_sum;
+    }
     // Stages: enough bytes in flight to cover the HBM latency at an SM's share of the bandwidth (about 48 KB), and at
     // least three when they fit (a warp may hold two stages while it carries rows over).
-    const int stage_bytes = kFastT * row_bytes;
+    const int null_bytes = kFastT / 8 * ((a.knull0 != nullptr) + (a.vnull != nullptr) + (a.pnull != nullptr));
+    const int stage_bytes = kFastT * row_bytes + null_bytes;
     int NS = static_cast<int>(env_int("QDB_FAST_STAGES", stage_bytes <= 16 * 1024 ? 4 : (stage_bytes <= 40 * 1024 ? 3 : 2)));
     NS = std::min(6, std::max(2, NS));
     // Compressed keys take each stage's key slots plus 64 bytes: a group is copied from the 16-byte boundary below
@@ -371,21 +388,44 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
         sl.pred = off;
         off += NS * kFastT * ps;
     }
+    if (ms) {
+        sl.mask = off;
+        off += NS * kFastT;
+    }
+    for (auto& c : {std::make_pair(a.knull0, &sl.knull0), std::make_pair(a.vnull, &sl.vnull), std::make_pair(a.pnull, &sl.pnull)})
+        if (c.first) {
+            *c.second = off;
+            off += NS * (kFastT / 8);
+        }
     sl.bytes = stage_bytes;
 
     const bool has_mm = a.has_min || a.has_max;
-    const size_t slot_bytes = 8 + 4 + (a.has_sum ? 8 : 0) + (has_mm ? (vk_is_32(vk) ? 8 : 16) : 0);
+    const size_t slot_bytes = 8 + 4 + (a.has_sum ? (a.wide ? 12 : 8) : 0) + (has_mm ? (vk_is_32(vk) ? 8 : 16) : 0);
     const size_t bucket_bytes = 2 * slot_bytes;
-    auto layout_table = [&](AggArgs& x, int NB) {  // offsets of the table arrays; returns the bytes used
+    auto layout_table = [&](AggArgs& x, int NB, int rep) {  // offsets of the table arrays; returns the bytes used
         const size_t S = static_cast<size_t>(NB) * 2;
+        const size_t E = S << rep;  // states
         size_t o = 0;
         x.NB = NB;
+        x.rep_shift = rep;
         x.so_keys = static_cast<int32_t>(o); o += S * 8;
-        x.so_mn = static_cast<int32_t>(o); o += has_mm ? S * (vk_is_32(vk) ? 8 : 16) : 0;
-        x.so_cnt = static_cast<int32_t>(o); o += S * 4;
-        x.so_l0 = static_cast<int32_t>(o); o += a.has_sum ? S * 4 : 0;
-        x.so_l1 = static_cast<int32_t>(o); o += a.has_sum ? S * 4 : 0;
+        x.so_mn = static_cast<int32_t>(o); o += has_mm ? E * (vk_is_32(vk) ? 8 : 16) : 0;
+        x.so_cnt = static_cast<int32_t>(o); o += E * 4;
+        x.so_l0 = static_cast<int32_t>(o); o += a.has_sum ? E * 4 : 0;
+        x.so_l1 = static_cast<int32_t>(o); o += a.has_sum ? E * 4 : 0;
+        x.so_l2 = static_cast<int32_t>(o); o += a.wide ? E * 4 : 0;
         return (o + 127) & ~size_t(127);
+    };
+    // Copies of every state of a table of NB buckets that `rows` rows go to, in `bytes` of shared memory: as many as
+    // fit, at most one per lane and kMaxStates in all, and no more than half the rows (each copy is cleared and merged).
+    auto rep_of = [&](int NB, int64_t rows, size_t bytes) {
+        const size_t S = static_cast<size_t>(NB) * 2;
+        const int cap = static_cast<int>(env_int("QDB_REP_MAX", 5));
+        int rep = 0;
+        while (rep < cap && (S << (rep + 1)) <= kMaxStates && static_cast<int64_t>(S << (rep + 1)) <= rows / 2 &&
+               S * 8 + (S << (rep + 1)) * (slot_bytes - 8) + 128 <= bytes)
+            ++rep;
+        return rep;
     };
 
     // Spill plan: partitions small enough for the spill pass's table (one CTA per SM, the largest table shared
@@ -435,8 +475,9 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
     const size_t list_bytes = static_cast<size_t>(kFastWarps) * kListCap * 2;
     const size_t spill_words_bytes =
         spill_bits >= 0 ? ((size_t(4) << spill_bits) + kSeenWords * 4 + 127) & ~size_t(127) : 0;
+    const size_t touch_bytes = a.nul ? static_cast<size_t>(kFastWarps) * kTouchCap * 8 : 0;
     const size_t budget = static_cast<size_t>(di.max_smem_optin) - 1024 - ring - bar_bytes - list_bytes -
-                          spill_words_bytes;
+                          spill_words_bytes - touch_bytes;
     int NBmax = static_cast<int>(budget / bucket_bytes);
     const int64_t forced = env_int("QDB_FAST_BUCKETS", 0);
     if (forced > 0 && forced < NBmax) NBmax = static_cast<int>(forced);
@@ -445,12 +486,12 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
     // otherwise the largest table that fits, with the misses spilled by key hash.
     const uint64_t groups = static_cast<uint64_t>(gb->capacity) + 1;
     const bool fits = groups <= static_cast<uint64_t>(NBmax);
-    const int NB = fits ? static_cast<int>(std::max<uint64_t>(64, std::min<uint64_t>(NBmax, 2 * groups))) : NBmax;
+    const int NB = fits ? static_cast<int>(std::max<uint64_t>(16, std::min<uint64_t>(NBmax, 2 * groups))) : NBmax;
     if (fits) spill_bits = -1;
-    const size_t tab_bytes = layout_table(a, NB);
+    const int64_t cta_rows = (a.n + ctas_plan - 1) / ctas_plan;
+    const size_t tab_bytes = layout_table(a, NB, fits ? rep_of(NB, cta_rows, budget) : 0);
     a.fits = fits ? 1 : 0;
-    a.probe_b = fits ? 8 : 1;
-    a.dedup = static_cast<int32_t>(env_int("QDB_DEDUP", 2));
+    a.probe_b = fits ? std::min(kProbeBuckets, NB) : 1;
     a.flush_rounds = static_cast<int32_t>(env_int("QDB_FLUSH_ROUNDS", 16));
     a.T = kFastT;
     a.NS = NS;
@@ -492,7 +533,8 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
     a.so_bar = static_cast<int32_t>(tab_bytes);
     a.so_list = static_cast<int32_t>(tab_bytes + bar_bytes);
     a.so_spill = static_cast<int32_t>(a.so_list + list_bytes);
-    a.so_stage = static_cast<int32_t>(a.so_spill + spill_words_bytes);
+    a.so_touch = static_cast<int32_t>(a.so_spill + spill_words_bytes);
+    a.so_stage = static_cast<int32_t>(a.so_touch + touch_bytes);
     const size_t smem = a.so_stage + ring;
     *used = true;
     int32_t rc = launch_fast(gb, a, ptype, smem, s);
@@ -504,12 +546,12 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
     // partition is cut into slices only when there are fewer partitions than CTAs.  Over the first of two levels the
     // table takes a key only into its home bucket and sends the rest on; the last level's table takes every key.
     AggArgs b = a;
-    const size_t tab2 = layout_table(b, NB2);
+    const size_t tab2 = layout_table(b, NB2, 0);
     b.so_spill = static_cast<int32_t>(tab2);  // the prefix of the cell fills
     b.so_spill2 = static_cast<int32_t>(tab2 + prefix2);
     const size_t smem2 = tab2 + prefix2 + fill2_bytes;
     b.fits = spill_bits2 ? 0 : 1;
-    b.probe_b = spill_bits2 ? 1 : 8;
+    b.probe_b = spill_bits2 ? 1 : std::min(kProbeBuckets, NB2);
     const int64_t parts = int64_t(1) << spill_bits;
     const int64_t ctas2 = static_cast<int64_t>(di.sm_count);
     const int64_t slices = std::max<int64_t>(1, std::min<int64_t>(a.spill_ctas, ctas2 / parts));
@@ -526,7 +568,7 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
         c.spill2_fill = nullptr;
         c.spill2_bits = 0;
         c.fits = 1;
-        c.probe_b = 8;
+        c.probe_b = std::min(kProbeBuckets, NB2);
         const int64_t items3 = int64_t(1) << c.spill_bits;
         rc = launch_fspill(gb, c, smem2, std::min<int64_t>(ctas2, items3), 1, s);
     }
@@ -695,12 +737,19 @@ static int32_t process_impl(qdb_gb* gb, const void* const* key_cols, const uint6
     a.counters = gb->counters;
     a.capacity = static_cast<unsigned long long>(gb->capacity);
     const bool nulls = a.knull0 || a.knull1 || a.vnull || a.pnull;
-    if (!nulls && !mask && gb->placement != QDB_PLACE_GLOBAL && n >= kFastT && env_int("QDB_AGG_FAST", 1) != 0 &&
+    // The fast pass takes calls of whole tiles and aligned columns.  NULL masks and a row mask are staged beside the
+    // columns in instantiations of their own (a single key column: a composite key with a NULL component lives in
+    // the table's second region, which only the general pass fills).
+    const bool masked = nulls || mask;
+    if (gb->placement != QDB_PLACE_GLOBAL && n >= kFastT && env_int("QDB_AGG_FAST", 1) != 0 &&
+        (!masked || (!kz && !km && gb->n_key_cols == 1)) &&
         (kz || aligned16(a.key0)) && (!a.key1 || aligned16(a.key1)) && (!a.vals || aligned16(a.vals)) &&
-        (!a.pcol || aligned16(a.pcol))) {
+        (!a.pcol || aligned16(a.pcol)) && aligned16(a.knull0) && aligned16(a.vnull) && aligned16(a.pnull) && aligned16(mask)) {
         bool used = false;
+        a.nul = masked ? 1 : 0;
         const int32_t rc = process_fast(gb, a, pred, ptype, s, &used);
         if (rc != QDB_OK || used) return rc;
+        a.nul = 0;
     }
     if (kz || km) return kNotFused;
 

@@ -100,7 +100,14 @@ struct AggArgs {
     int32_t so_tags = 0, so_keys = 0;
     int32_t fits = 0;      // 1: every group fits the table: a key may overflow into the next probe_b - 1 buckets
     int32_t probe_b = 1;   // buckets a claim may visit
-    int32_t dedup = 2;     // warp aggregation of equal keys: 0 off, 1 on, 2 decided per warp from its first batches
+    // Calls of the fast pass with NULL masks or a row mask: the predicate's type (0 none), whether a key may be NULL, sums
+    // of doubles in 96 bits (a third limb at so_l2), and the warps' queues of keys to look up.
+    int32_t nul = 0;
+    int32_t ptype = 0;
+    int32_t null_keys = 0;
+    int32_t wide = 0;
+    int32_t so_touch = 0;
+    int32_t rep_shift = 0; // 2^rep_shift copies of every slot's state (tables of few groups)
     int32_t pred_float = 0;  // the fast pass compares IEEE predicate values as order-preserving integers
     int32_t flush_rounds = 16;  // lock-step probe rounds of a shared table's merge into the global table
     // Second spill level (fast pass, tables with more partitions than one pass writes well): the spill pass over the

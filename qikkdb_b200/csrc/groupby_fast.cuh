@@ -1,5 +1,5 @@
-// The fast form of the fused filter + hash-aggregate pass, for the common call: no NULL masks, no precomputed
-// mask, 16-byte aligned columns (the replacement of kernel_filter -> reconstructColKeep -> group_by_kernel,
+// The fast form of the fused filter + hash-aggregate pass, for calls of 16-byte aligned columns that hold a whole tile
+// (the replacement of kernel_filter -> reconstructColKeep -> group_by_kernel,
 // qikkDB/QueryEngine/GPUCore/GPUFilter.cuh:22-44, GPUReconstruct.cuh:272-355, GPUGroupBy.cuh:68-196, and of the
 // multi-key kernel_group_by_multi_key, GPUGroupByMultiKey.cuh:156-259, for (int32, int32) keys).
 //
@@ -16,9 +16,8 @@
 //     improves on the slot's bound.  Integer sums wrap like the reference's 64-bit atomicAdd; float and double
 //     values are added in fixed point (q = v * 2^F, F from the CTA's first tile and its row count, so that no sum
 //     can overflow), exactly for float values; values outside that window take the FP64 global path;
-//   * when equal keys are common within a warp (few groups, or heavy skew), lanes holding one slot are combined
-//     first (__match_any_sync on the slot, then full-warp __reduce_*_sync of the group's count, sum pieces and
-//     min/max, one round per group of four or more lanes), and one lane updates the slot;
+//   * a table of few groups keeps up to 32 copies of every slot's state, one per lane, so that lanes of a warp that
+//     meet on one key update different words (the copies are added up when the table is merged);
 //   * a miss is appended to its partition's cell of the hash-partitioned spill area (gb_fspill_kernel aggregates
 //     each partition in shared memory afterwards) or, without one, inserted into the global table.
 // At the end every CTA merges its table into the global open-addressing table.
@@ -33,10 +32,15 @@ constexpr int kFastThreads = (kFastWarps + 1) * 32; // + one producer warp
 constexpr int kFastSeg = 4;                         // 32-row segments per warp and tile
 constexpr int kFastR = 32 * kFastSeg;               // rows per warp and tile
 constexpr int kFastT = kFastWarps * kFastR;         // rows per tile (2048)
-constexpr int kDedupTrial = 4;                      // steps a warp runs with warp aggregation before deciding
-constexpr int kDedupGroup = 4;                      // lanes sharing a slot that are combined before the update
 constexpr int kMaxSpillBits = 13;                   // partitions the aggregation pass writes: at most 8192
 constexpr int kMaxSpill2Bits = 6;                   // second-level partitions per first-level one: at most 64
+// The NULL key's word in the shared tables and the spill (the global table has a slot of its own for it).  A real key
+// with this word is never put there: it goes to the global table.
+constexpr uint64_t kNullWord = kEmpty + 1;
+constexpr int kTouchCap = 64;                       // queued keys per warp (FM_NULL)
+// Buckets a key may be placed in where a table holds every group (a key that finds no place takes the global table for
+// every row).
+constexpr int kProbeBuckets = 64;
 constexpr uint64_t kHashMul = 0x9E3779B97F4A7C15ull;
 
 __device__ __forceinline__ uint32_t atoms_or(uint32_t a, uint32_t x) {
@@ -51,30 +55,46 @@ __device__ __forceinline__ void lds128(uint32_t a, uint64_t& k0, uint64_t& k1) {
 // Shared-window addresses of the bucketed table's arrays.  A bucket is two slots whose key words sit side by side
 // (keys[2 b + j]); the slot's state lives in position-major arrays at index s = j NB + b, so that the states of
 // different buckets' first positions fall in consecutive banks.
+//
+// A table of few groups keeps 2^rep_shift copies of every state (slot s, copy r at index (s << rep_shift) + r); lane l
+// of every warp updates copy l mod 2^rep_shift and the merge adds the copies up.
 struct FTab {
-    uint32_t keys, cnt, l0, l1, mm;
+    uint32_t keys, cnt, l0, l1, l2, mm;  // state arrays: the address of this lane's copy of slot 0
     uint32_t NB;
+    uint32_t osh;                    // slot s's 4-byte state is at s << osh
 };
 
+template <typename VT>
 __device__ __forceinline__ FTab ftab(unsigned char* sm, const AggArgs& a) {
     FTab t;
+    const uint32_t r = threadIdx.x & ((1u << a.rep_shift) - 1u);
     t.keys = smem_u32(sm + a.so_keys);
-    t.cnt = smem_u32(sm + a.so_cnt);
-    t.l0 = smem_u32(sm + a.so_l0);
-    t.l1 = smem_u32(sm + a.so_l1);
-    t.mm = smem_u32(sm + a.so_mn);
+    t.cnt = smem_u32(sm + a.so_cnt) + r * 4u;
+    t.l0 = smem_u32(sm + a.so_l0) + r * 4u;
+    t.l1 = smem_u32(sm + a.so_l1) + r * 4u;
+    t.l2 = smem_u32(sm + a.so_l2) + r * 4u;
+    t.mm = smem_u32(sm + a.so_mn) + r * (sizeof(VT) == 4 ? 8u : 16u);
     t.NB = static_cast<uint32_t>(a.NB);
+    t.osh = 2u + static_cast<uint32_t>(a.rep_shift);
     return t;
 }
 
 // Hash of a key word for the shared tables and the spill: one 64-bit multiply (Fibonacci hashing, Knuth TAOCP vol. 3,
 // 6.4).  Its top bits pick the spill partition, the 32 bits below bit `shift` (32 - partition bits) the bucket (so
 // a partition's rows spread over every bucket of the spill pass's table), and bits 32..46 the bit of the seen-once
-// filter.  The global table hashes with the independent mix64.
+// filter.  The global table hashes with the independent mix64.  Being linear it spreads dense and evenly spaced keys
+// better than chance (no full buckets at half load, against 7-10 % with a mixing hash, which made the spill pass of
+// 16.8M composite groups 4.2 instead of 3.8 ms), at the price of strides that it lines up: see falt.
 __device__ __forceinline__ uint64_t fhash(uint64_t kw) { return kw * kHashMul; }
 __device__ __forceinline__ uint32_t fbucket(uint64_t m, int shift, uint32_t NB) {
     const uint32_t x = __funnelshift_rc(static_cast<uint32_t>(m), static_cast<uint32_t>(m >> 32), shift);
     return __umulhi(x, NB);
+}
+
+// The bucket a key whose home bucket is full tries next, from other bits of its hash: home buckets that an unlucky stride
+// of the keys lines up would also fill their neighbours.
+__device__ __forceinline__ uint32_t falt(uint64_t m, uint32_t NB) {
+    return __umulhi((static_cast<uint32_t>(m) ^ static_cast<uint32_t>(m >> 32)) * 0x9E3779B1u, NB);
 }
 
 // Looks kw up in bucket b: returns its slot or -1; empty: the bucket has a free position.
@@ -85,11 +105,12 @@ __device__ __forceinline__ int fprobe(const FTab& t, uint32_t b, uint64_t kw, bo
     return (k0 == kw) ? static_cast<int>(b) : ((k1 == kw) ? static_cast<int>(t.NB + b) : -1);
 }
 
-// Finds or claims kw in buckets b, b + 1, ... (nb buckets at most): a new key is claimed with a CAS on its key word.
-// Returns the slot or -1.
+// Finds or claims kw in bucket b, then in its second bucket and those after it (nb buckets in all): a new key is claimed
+// with a CAS on its key word.  Returns the slot or -1.
 static __device__ __noinline__ int fclaim(const FTab t, uint32_t b, uint64_t kw, int nb) {
     uint32_t bb = b;
     for (int k = 0; k < nb; ++k) {
+        if (k == 1) bb = falt(fhash(kw), t.NB);
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const uint32_t ka = t.keys + (bb * 2u + j) * 8u;
@@ -100,7 +121,7 @@ static __device__ __noinline__ int fclaim(const FTab t, uint32_t b, uint64_t kw,
                 if (prev == kEmpty || prev == kw) return static_cast<int>(j * t.NB + bb);
             }
         }
-        bb = (bb + 1u == t.NB) ? 0u : bb + 1u;
+        if (k) bb = (bb + 1u == t.NB) ? 0u : bb + 1u;
     }
     return -1;
 }
@@ -111,6 +132,8 @@ static __device__ __noinline__ int fclaim(const FTab t, uint32_t b, uint64_t kw,
 // (|v| < 2^emax) of the CTA's first tile; values up to 2^(emax + 2) are kept.
 //   float: q = m24 << sh with sh = biased exponent - sh0 in [0, 39 - hb]: exact.
 //   double: q = round(v * 2^F) for |v| in [lo, hi): every kept value has at least 24 significant bits.
+// FM_WIDE keeps doubles in 96 bits (three limbs), so that addends need no headroom: q = round(v * 2^(61 - emax)) for |v|
+// below 2^(emax + 2), every bit of a value down to 2^(emax - 9) and at least 40 bits of any kept one.
 // ---------------------------------------------------------------------------------------------
 struct FixQ {
     int sh0 = 0;
@@ -121,12 +144,19 @@ struct FixQ {
     double hi = 0.0;
 };
 
-template <typename VT>
+template <typename VT, bool WIDE>
 __device__ __forceinline__ FixQ fixq(int emax, int hb) {
     FixQ f;
     emax = max(-900, min(900, emax));
+    if constexpr (WIDE) {
+        f.scale = ldexp(1.0, 61 - emax);
+        f.inv = ldexp(1.0, emax - 61);
+        f.lo = ldexp(1.0, emax - 22);
+        f.hi = ldexp(1.0, emax + 2);
+        return f;
+    }
     const int g = 2;
-    f.shmax = max(0, 39 - hb);
+    f.shmax = max(0, min(30, 39 - hb));
     if constexpr (std::is_same<VT, float>::value) {
         // A value of exponent emax + g would take sh = shmax.  sh0 stays in [1, 254 - shmax], so the biased exponents
         // 0 (zero, subnormals) and 255 (Inf, NaN) always fall outside [sh0, sh0 + shmax].
@@ -150,9 +180,10 @@ __device__ __forceinline__ long long addq(VT v, const FixQ& f, bool& ok) {
         const uint32_t sh = ((b >> 23) & 0xffu) - static_cast<uint32_t>(f.sh0);  // below sh0: wraps to a large value
         const bool inw = sh <= static_cast<uint32_t>(f.shmax);
         ok = inw | ((b << 1) == 0u);  // zero is exact; subnormals, NaN and Inf take the FP64 path
-        const uint64_t mag = inw ? static_cast<uint64_t>((b & 0x7fffffu) | 0x800000u) << sh : 0ull;
-        const uint64_t sg = static_cast<uint64_t>(static_cast<int64_t>(static_cast<int32_t>(b) >> 31));
-        return static_cast<long long>((mag ^ sg) - sg);
+        const int32_t sg = static_cast<int32_t>(b) >> 31;
+        const int32_t m = static_cast<int32_t>(((b & 0x7fffffu) | 0x800000u) ^ static_cast<uint32_t>(sg)) - sg;
+        // one widening multiply shifts and sign-extends (sh is at most shmax <= 30: hb is at least 9)
+        return static_cast<long long>(inw ? m : 0) * static_cast<long long>(static_cast<int32_t>(1u << (sh & 31u)));
     } else if constexpr (std::is_same<VT, double>::value) {
         const double m = fabs(v);
         ok = (m == 0.0) | ((m >= f.lo) & (m < f.hi));  // false for NaN and Inf
@@ -170,7 +201,7 @@ __device__ __forceinline__ int fexp(VT v) { return value_exp<VT>(v); }
 // ---------------------------------------------------------------------------------------------
 // Table initialisation and merge into the global table.
 // ---------------------------------------------------------------------------------------------
-template <typename VT>
+template <typename VT, bool WIDE>
 __device__ __forceinline__ void ftab_init(unsigned char* sm, const AggArgs& a, int tid, int nthreads) {
     const int S = a.NB * 2;
     uint64_t* keys = reinterpret_cast<uint64_t*>(sm + a.so_keys);
@@ -179,12 +210,14 @@ __device__ __forceinline__ void ftab_init(unsigned char* sm, const AggArgs& a, i
     unsigned* l1 = reinterpret_cast<unsigned*>(sm + a.so_l1);
     unsigned long long* mm = reinterpret_cast<unsigned long long*>(sm + a.so_mn);
     const bool has_mm = a.has_min || a.has_max;
-    for (int i = tid; i < S; i += nthreads) {
-        keys[i] = kEmpty;
+    for (int i = tid; i < S; i += nthreads) keys[i] = kEmpty;
+    const int E = S << a.rep_shift;
+    for (int i = tid; i < E; i += nthreads) {
         cnt[i] = 0u;
         if (a.has_sum) {
             l0[i] = 0u;
             l1[i] = 0u;
+            if (WIDE) reinterpret_cast<unsigned*>(sm + a.so_l2)[i] = 0u;
         }
         if (has_mm) {
             if (sizeof(VT) == 4) {
@@ -203,7 +236,7 @@ __device__ __forceinline__ void ftab_init(unsigned char* sm, const AggArgs& a, i
 // after a.flush_rounds rounds (a long probe run) finishes with the one-key search, which bounds the probe and reports
 // a full table.
 
-template <typename VT>
+template <typename VT, bool WIDE>
 __device__ __forceinline__ void ftab_flush(unsigned char* sm, const AggArgs& a, const FixQ& fq,
                                            unsigned long long* claims) {
     constexpr bool V32 = sizeof(VT) == 4;
@@ -214,6 +247,7 @@ __device__ __forceinline__ void ftab_flush(unsigned char* sm, const AggArgs& a, 
     const unsigned* cnt = reinterpret_cast<const unsigned*>(sm + a.so_cnt);
     const unsigned* l0 = reinterpret_cast<const unsigned*>(sm + a.so_l0);
     const unsigned* l1 = reinterpret_cast<const unsigned*>(sm + a.so_l1);
+    const unsigned* l2 = reinterpret_cast<const unsigned*>(sm + a.so_l2);
     const unsigned char* mm = sm + a.so_mn;
     const uint64_t mask = a.main.mask;
     constexpr int U = 4;
@@ -226,7 +260,11 @@ __device__ __forceinline__ void ftab_flush(unsigned char* sm, const AggArgs& a, 
             const int ki = i0 + u * blockDim.x;
             key[u] = (ki < S) ? keys[ki] : kEmpty;
             g[u] = nullptr;
-            pend[u] = key[u] != kEmpty && cnt[(ki & 1) * a.NB + (ki >> 1)] != 0u;  // key index 2 b + j -> state j NB + b
+            pend[u] = key[u] != kEmpty;
+            if (a.null_keys && key[u] == kNullWord) {
+                g[u] = g_special(a.main, W, 0, claims);
+                pend[u] = false;
+            }
             pos[u] = pend[u] ? home_slot(a.main, mix64(key[u])) : 0ull;
         }
 #pragma unroll
@@ -261,29 +299,39 @@ __device__ __forceinline__ void ftab_flush(unsigned char* sm, const AggArgs& a, 
             if (pend[u]) g[u] = g_find_from(a.main, W, key[u], pos[u], cur[u], a.counters, claims);
             if (!g[u]) continue;
             const int ki = i0 + u * blockDim.x;
-            const int i = (ki & 1) * a.NB + (ki >> 1);
-            const unsigned long long c = cnt[i];
-            uint64_t sumbits = 0;
-            if (a.has_sum) {
-                const uint64_t s = (static_cast<uint64_t>(l1[i]) << 32) | l0[i];
-                if (VFLOAT) {
-                    const double d = static_cast<double>(static_cast<long long>(s)) * fq.inv;
-                    memcpy(&sumbits, &d, 8);
-                } else {
-                    sumbits = s;
+            const int i = ((ki & 1) * a.NB + (ki >> 1)) << a.rep_shift;  // key index 2 b + j -> state j NB + b
+            unsigned long long c = 0;
+            uint64_t sum = 0;
+            __int128 wide = 0;
+            long long mn = V32 ? INT_MAX : LLONG_MAX, mx = V32 ? INT_MIN : LLONG_MIN;
+#pragma unroll 1
+            for (int k = 0; k < 1 << a.rep_shift; ++k) {
+                // lanes start at different copies, so the copies of neighbouring slots are read from different banks
+                const int e = i + ((k + static_cast<int>(threadIdx.x)) & ((1 << a.rep_shift) - 1));
+                c += cnt[e];
+                if (a.has_sum) {
+                    const uint64_t lo = (static_cast<uint64_t>(l1[e]) << 32) | l0[e];
+                    if (WIDE) wide += (static_cast<__int128>(static_cast<int32_t>(l2[e])) << 64) + static_cast<__int128>(lo);
+                    else sum += lo;
+                }
+                if (a.has_min || a.has_max) {
+                    if (V32) {
+                        const int* w = reinterpret_cast<const int*>(mm) + 2 * e;
+                        mn = min(mn, static_cast<long long>(w[0]));
+                        mx = max(mx, static_cast<long long>(w[1]));
+                    } else {
+                        const long long* w = reinterpret_cast<const long long*>(mm) + 2 * e;
+                        mn = min(mn, w[0]);
+                        mx = max(mx, w[1]);
+                    }
                 }
             }
-            long long mn = 0, mx = 0;
-            if (a.has_min || a.has_max) {
-                if (V32) {
-                    const int* w = reinterpret_cast<const int*>(mm) + 2 * i;
-                    mn = w[0];
-                    mx = w[1];
-                } else {
-                    const long long* w = reinterpret_cast<const long long*>(mm) + 2 * i;
-                    mn = w[0];
-                    mx = w[1];
-                }
+            uint64_t sumbits = sum;
+            if (a.has_sum && VFLOAT) {
+                const double d = (WIDE ? limbs96_to_double(static_cast<unsigned>(wide), static_cast<unsigned>(wide >> 32),
+                                                           static_cast<unsigned>(wide >> 64))
+                                       : static_cast<double>(static_cast<long long>(sum))) * fq.inv;
+                memcpy(&sumbits, &d, 8);
             }
             g_merge(g[u], a.L, a.has_sum, a.has_min, a.has_max, V32, VFLOAT, c, sumbits, mn, mx);
         }
@@ -299,6 +347,8 @@ constexpr int FM_SUM = 1;
 constexpr int FM_MM = 2;
 constexpr int FM_VALS = 4;
 constexpr int FM_KZ = 8;  // the key column is an AAFL-compressed block (single key, not DOUBLE)
+constexpr int FM_NULL = 32;  // NULL masks (key, value, predicate) or a row mask; the predicate type is read at run time
+constexpr int FM_WIDE = 64;  // 96-bit sums of doubles
 constexpr int FM_KMOD = 16;  // keys are replaced by key % m as they are read (single INT32 or INT64 key)
 
 template <typename VT, int MODE>
@@ -306,6 +356,8 @@ struct FastWarp {
     static constexpr bool SUM = (MODE & FM_SUM) != 0;
     static constexpr bool MM = (MODE & FM_MM) != 0;
     static constexpr bool VALS = (MODE & FM_VALS) != 0;
+    static constexpr bool NUL = (MODE & FM_NULL) != 0;
+    static constexpr bool WIDE = (MODE & FM_WIDE) != 0;
     const AggArgs& a;
     FTab t;
     FixQ fq;
@@ -315,10 +367,7 @@ struct FastWarp {
     bool fits = false;
     bool use_smem = true;  // probe the shared table at all
     bool spill_ok = false; // append misses to the spill area
-    bool dedup = false;
     bool counting = true;  // count lookups and hits (until the warp has judged its hit rate)
-    int trial = 0;         // steps run so far in the warp-aggregation trial
-    unsigned trial_hits = 0, trial_leaders = 0;  // warp totals over the trial
     unsigned hits = 0, tries = 0;
     // Where a miss goes: partition q = (fhash(key) >> part_shift) & part_mask, appended to cell cell_base + q cell_mul
     // of spill_out (records of 16 bytes, or 8 for a count-only table) at the position its shared fill counter
@@ -328,106 +377,83 @@ struct FastWarp {
     unsigned cell_cap = 0;
     int part_shift = 64;
     uint32_t part_mask = 0;
-    int64_t cell_base = 0;
-    int64_t cell_mul = 0;
+    uint32_t cell_base = 0;
+    uint32_t cell_mul = 0;
     uint64_t* spill_out = nullptr;
+    // Keys of rows with a NULL value that missed the table (they only have to exist in the global table), looked up 32
+    // at a time.
+    uint64_t* touch = nullptr;
+    int touched = 0;
 
     __device__ __forceinline__ FastWarp(const AggArgs& args, const FTab& tab, const FixQ& f, unsigned long long* c)
         : a(args), t(tab), fq(f), claims(c) {}
 
-    __device__ __forceinline__ void global_row(uint64_t kw, VT v) {
+    // One row into the global table; esc: kw is a real key although it is the NULL key's word; vn: its value is NULL.
+    __device__ __forceinline__ void global_row(uint64_t kw, VT v, bool esc = false, bool vn = false) {
         uint64_t* slot = (kw == kEmpty) ? g_special(a.main, a.L.W, 1, claims)
-                                        : g_find(a.main, a.L.W, kw, mix64(kw), a.counters, claims);
-        if (slot) {
+                         : (a.null_keys && kw == kNullWord && !esc)
+                             ? g_special(a.main, a.L.W, 0, claims)
+                             : g_find(a.main, a.L.W, kw, mix64(kw), a.counters, claims);
+        if (slot && !vn) {
             if (VALS) g_acc_row<VT>(slot, a, v);
             else g_count_row(slot, a.L);
         }
     }
 
-    // Adds (n rows, sum addend q, encoded min e_mn and max e_mx) to slot s.
-    __device__ __forceinline__ void update(uint32_t s, unsigned n, long long q, long long e_mn, long long e_mx) {
-        reds_add(t.cnt + s * 4u, n);
+    __device__ __forceinline__ void touch_queue(bool put, uint64_t kw, unsigned lane) {
+        const unsigned b = __ballot_sync(0xffffffffu, put);
+        if (b == 0u) return;
+        if (put) touch[touched + __popc(b & ((1u << lane) - 1u))] = kw;
+        touched += __popc(b);
+        if (touched > kTouchCap - 32) touch_drain(lane, 32);
+    }
+    // Looks up the last `n` queued keys (at most 32).
+    __device__ __forceinline__ void touch_drain(unsigned lane, int n) {
+        __syncwarp();
+        touched -= n;
+        if (static_cast<int>(lane) < n) global_row(touch[touched + lane], VT{}, false, true);
+        __syncwarp();
+    }
+
+    // Adds one row (its sum addend q, its value v) to slot s.
+    __device__ __forceinline__ void update(uint32_t s, long long q, VT v) {
+        const uint32_t o = s << t.osh;
+        reds_add(t.cnt + o, 1u);
         if constexpr (SUM) {
             const unsigned long long uq = static_cast<unsigned long long>(q);
             const unsigned x0 = static_cast<unsigned>(uq);
-            const unsigned old0 = atoms_add(t.l0 + s * 4u, x0);
+            const unsigned old0 = atoms_add(t.l0 + o, x0);
             const unsigned c = (old0 + x0 < old0) ? 1u : 0u;
-            reds_add(t.l1 + s * 4u, static_cast<unsigned>(uq >> 32) + c);
+            if constexpr (WIDE) {
+                const unsigned long long y1 = (uq >> 32) + c;
+                const unsigned x1 = static_cast<unsigned>(y1);
+                const unsigned old1 = atoms_add(t.l1 + o, x1);
+                const unsigned y2 = (q < 0 ? 0xffffffffu : 0u) + static_cast<unsigned>(y1 >> 32) + ((old1 + x1 < old1) ? 1u : 0u);
+                if (y2) reds_add(t.l2 + o, y2);
+            } else {
+                reds_add(t.l1 + o, static_cast<unsigned>(uq >> 32) + c);
+            }
         }
         if constexpr (MM) {
             if constexpr (sizeof(VT) == 4) {
-                const uint32_t w = t.mm + s * 8u;
+                const int32_t e = enc32(v);
+                const uint32_t w = t.mm + o * 2u;
                 const uint64_t cur = lds64(w);
-                if (a.has_min && static_cast<int32_t>(e_mn) < static_cast<int32_t>(cur)) reds_min32(w, static_cast<int32_t>(e_mn));
-                if (a.has_max && static_cast<int32_t>(e_mx) > static_cast<int32_t>(cur >> 32)) reds_max32(w + 4u, static_cast<int32_t>(e_mx));
+                if (a.has_min && e < static_cast<int32_t>(cur)) reds_min32(w, e);
+                if (a.has_max && e > static_cast<int32_t>(cur >> 32)) reds_max32(w + 4u, e);
             } else {
-                const uint32_t w = t.mm + s * 16u;
-                if (a.has_min && e_mn < lds64s(w)) reds_min64(w, e_mn);
-                if (a.has_max && e_mx > lds64s(w + 8u)) reds_max64(w + 8u, e_mx);
+                const long long e = enc64(v);
+                const uint32_t w = t.mm + o * 4u;
+                if (a.has_min && e < lds64s(w)) reds_min64(w, e);
+                if (a.has_max && e > lds64s(w + 8u)) reds_max64(w + 8u, e);
             }
         }
-    }
-
-    __device__ __forceinline__ long long encv(VT v) const {
-        if constexpr (sizeof(VT) == 4) return enc32(v);
-        else return enc64(v);
-    }
-
-    // Warp aggregation of one row per lane: lanes holding one slot in groups of kDedupGroup or more are combined with
-    // full-warp reductions (one round per such group) and one lane updates the slot; other hit lanes update directly.
-    __device__ __forceinline__ void dedup_rows(bool hit, int slot, long long q, VT v, unsigned lane) {
-        const long long e = MM ? encv(v) : 0;
-        const unsigned peers = __match_any_sync(0xffffffffu, hit ? static_cast<unsigned>(slot) : (0x80000000u | lane));
-        const bool big = hit && __popc(peers) >= kDedupGroup;
-        unsigned bigmask = __ballot_sync(0xffffffffu, big);
-        if (trial < kDedupTrial) {
-            trial_hits += __popc(__ballot_sync(0xffffffffu, hit));
-            trial_leaders += __popc(__ballot_sync(0xffffffffu, hit && (__ffs(peers) - 1 == static_cast<int>(lane))));
-        }
-        while (bigmask) {
-            const int leader = __ffs(bigmask) - 1;
-            const unsigned grp = __shfl_sync(0xffffffffu, peers, leader);
-            const bool in = (grp >> lane) & 1u;
-            long long qs = 0;
-            if constexpr (SUM) {
-                const unsigned uq0 = in ? static_cast<unsigned>(q) : 0u;
-                const unsigned s_lo = __reduce_add_sync(0xffffffffu, uq0 & 0xffffu);
-                const unsigned s_mid = __reduce_add_sync(0xffffffffu, uq0 >> 16);
-                const unsigned s_hi = __reduce_add_sync(
-                    0xffffffffu, in ? static_cast<unsigned>(static_cast<unsigned long long>(q) >> 32) : 0u);
-                qs = static_cast<long long>((static_cast<unsigned long long>(s_hi) << 32) +
-                                            (static_cast<unsigned long long>(s_mid) << 16) + s_lo);
-            }
-            long long g_mn = 0, g_mx = 0;
-            if constexpr (MM) {
-                if constexpr (sizeof(VT) == 4) {
-                    if (a.has_min) g_mn = __reduce_min_sync(0xffffffffu, in ? static_cast<int>(e) : INT_MAX);
-                    if (a.has_max) g_mx = __reduce_max_sync(0xffffffffu, in ? static_cast<int>(e) : INT_MIN);
-                } else {
-                    if (a.has_min) {
-                        const int h = __reduce_min_sync(0xffffffffu, in ? static_cast<int>(e >> 32) : INT_MAX);
-                        const unsigned l = __reduce_min_sync(
-                            0xffffffffu, (in && static_cast<int>(e >> 32) == h) ? static_cast<unsigned>(e) : 0xffffffffu);
-                        g_mn = static_cast<long long>((static_cast<unsigned long long>(static_cast<unsigned>(h)) << 32) | l);
-                    }
-                    if (a.has_max) {
-                        const int h = __reduce_max_sync(0xffffffffu, in ? static_cast<int>(e >> 32) : INT_MIN);
-                        const unsigned l = __reduce_max_sync(
-                            0xffffffffu, (in && static_cast<int>(e >> 32) == h) ? static_cast<unsigned>(e) : 0u);
-                        g_mx = static_cast<long long>((static_cast<unsigned long long>(static_cast<unsigned>(h)) << 32) | l);
-                    }
-                }
-            }
-            if (lane == static_cast<unsigned>(leader)) update(static_cast<uint32_t>(slot), __popc(grp), qs, g_mn, g_mx);
-            bigmask &= ~grp;
-        }
-        if (hit && !big) update(static_cast<uint32_t>(slot), 1u, q, e, e);
     }
 
     // Stores a spilled row as one record (key word, value bits: a single 8- or 16-byte store) at position pos of its
     // partition's cell.
     __device__ __forceinline__ void spill_store(uint64_t kw, VT v, uint32_t p, unsigned pos) {
-        const uint64_t idx = static_cast<uint64_t>(cell_base + static_cast<int64_t>(p) * cell_mul) * cell_cap + pos;
+        const uint32_t idx = (cell_base + p * cell_mul) * cell_cap + pos;  // an area holds fewer than 2^31 records
         if constexpr (VALS) {
             uint64_t vb = 0;
             memcpy(&vb, &v, sizeof(VT));
@@ -437,46 +463,60 @@ struct FastWarp {
         }
     }
 
-    // Two rows per lane: (act[u], kw[u], v[u]) for u = 0, 1.  The two rows' loads and arithmetic are independent, so
+    template <int U>
+    __device__ __forceinline__ void rows(const bool (&act)[U], const uint64_t (&kw)[U], const VT (&v)[U], unsigned lane) {
+        const bool no[U] = {};
+        rows<U>(act, kw, v, no, no, lane);
+    }
+
+    // U rows per lane: (act[u], kw[u], v[u]) (FM_NULL: vn[u] its value is NULL, esc[u] kw[u] is a real key
+    // that looks like the NULL key's word).  The rows' loads and arithmetic are independent, so
     // their latencies overlap; the rare paths (claims, next-bucket probes, misses) run under warp votes.
-    __device__ __forceinline__ void rows2(const bool (&act)[2], const uint64_t (&kw)[2], const VT (&v)[2], unsigned lane) {
-        long long q[2];
-        bool inwin[2], look[2], hit[2], empty[2];
-        uint64_t m[2], k0[2], k1[2];
-        uint32_t b[2];
-        int slot[2];
+    template <int U>
+    __device__ __forceinline__ void rows(const bool (&act)[U], const uint64_t (&kw)[U], const VT (&v)[U],
+                                         const bool (&vn)[U], const bool (&esc)[U], unsigned lane) {
+        long long q[U];
+        bool inwin[U], look[U], hit[U], empty[U];
+        uint64_t m[U], k0[U], k1[U];
+        uint32_t b[U];
+        int slot[U];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < U; ++u) {
             inwin[u] = true;
             q[u] = 0;
             if constexpr (SUM) q[u] = addq<VT>(v[u], fq, inwin[u]);
+            if constexpr (NUL) inwin[u] = inwin[u] | vn[u];
             m[u] = fhash(kw[u]);
             look[u] = act[u] & (kw[u] != kEmpty) & inwin[u] & use_smem;
+            if constexpr (NUL) look[u] = look[u] & !esc[u];
             b[u] = fbucket(m[u], bshift, t.NB);
             k0[u] = k1[u] = kEmpty;
         }
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
+        for (int u = 0; u < U; ++u)
             if (look[u]) lds128(t.keys + b[u] * 16u, k0[u], k1[u]);
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < U; ++u) {
             const bool h0 = k0[u] == kw[u];
             hit[u] = look[u] & (h0 | (k1[u] == kw[u]));
             slot[u] = hit[u] ? static_cast<int>(h0 ? b[u] : t.NB + b[u]) : -1;
             empty[u] = (k0[u] == kEmpty) | (k1[u] == kEmpty);
         }
         if (fits) {
-            // A table sized for every group places a key whose home bucket is full in a later bucket, almost always
-            // the next one: look there before the claim path.
-            bool nx[2];
+            // A table sized for every group places a key whose home bucket is full in its second bucket, or rarely in one
+            // after it: look there before the claim path.
+            bool nx[U], any_nx = false;
 #pragma unroll
-            for (int u = 0; u < 2; ++u) nx[u] = look[u] & !hit[u] & !empty[u];
-            if (__any_sync(0xffffffffu, nx[0] | nx[1])) {
+            for (int u = 0; u < U; ++u) {
+                nx[u] = look[u] & !hit[u] & !empty[u];
+                any_nx |= nx[u];
+            }
+            if (__any_sync(0xffffffffu, any_nx)) {
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
+                for (int u = 0; u < U; ++u) {
                     if (nx[u]) {
                         bool e2 = false;
-                        const int s2 = fprobe(t, (b[u] + 1u == t.NB) ? 0u : b[u] + 1u, kw[u], e2);
+                        const int s2 = fprobe(t, falt(m[u], t.NB), kw[u], e2);
                         if (s2 >= 0) {
                             slot[u] = s2;
                             hit[u] = true;
@@ -486,12 +526,15 @@ struct FastWarp {
             }
         }
         // Claim path: a new key with room in its bucket or (a table sized for every group) any key not found so far.
-        bool need[2];
+        bool need[U], any_need = false;
 #pragma unroll
-        for (int u = 0; u < 2; ++u) need[u] = look[u] & !hit[u] & (empty[u] | fits);
-        if (__any_sync(0xffffffffu, need[0] | need[1])) {
+        for (int u = 0; u < U; ++u) {
+            need[u] = look[u] & !hit[u] & (empty[u] | fits);
+            any_need |= need[u];
+        }
+        if (__any_sync(0xffffffffu, any_need)) {
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
+            for (int u = 0; u < U; ++u) {
                 bool go = need[u];
                 if (go && seen) {
                     // While a spilling table fills, a key is admitted on its second occurrence only, so that the
@@ -508,51 +551,45 @@ struct FastWarp {
         }
         if (counting) {
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
+            for (int u = 0; u < U; ++u) {
                 tries += look[u] ? 1u : 0u;
                 hits += hit[u] ? 1u : 0u;
             }
         }
-        if (dedup) {
 #pragma unroll
-            for (int u = 0; u < 2; ++u) dedup_rows(hit[u], slot[u], q[u], v[u], lane);
-            if (trial < kDedupTrial && ++trial == kDedupTrial && a.dedup == 2) {
-                const unsigned th = __reduce_add_sync(0xffffffffu, lane == 0 ? trial_hits : 0u);
-                const unsigned tl = __reduce_add_sync(0xffffffffu, lane == 0 ? trial_leaders : 0u);
-                dedup = th > 0 && (th - tl) * 2u >= th;  // keep it when half the hits share a slot with another lane
-            }
-        } else {
+        for (int u = 0; u < U; ++u)
+            if (hit[u] && !(NUL && vn[u])) update(static_cast<uint32_t>(slot[u]), q[u], v[u]);
+        bool miss[U], any_miss = false;
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                if (hit[u]) {
-                    const long long e = MM ? encv(v[u]) : 0;
-                    update(static_cast<uint32_t>(slot[u]), 1u, q[u], e, e);
-                }
-            }
+        for (int u = 0; u < U; ++u) {
+            miss[u] = act[u] & !hit[u];
+            any_miss |= miss[u];
         }
-        bool miss[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) miss[u] = act[u] & !hit[u];
-        if (__any_sync(0xffffffffu, miss[0] | miss[1])) {
-            // Both rows' spill positions are claimed before either record is stored, so the two shared-atomic round
+        if (__any_sync(0xffffffffu, any_miss)) {
+            // All rows' spill positions are claimed before any record is stored, so the shared-atomic round
             // trips overlap; rows that cannot spill (or whose cell is full) go to the global table.
-            bool sp[2];
-            unsigned pos[2];
-            uint32_t part[2];
+            bool sp[U];
+            unsigned pos[U];
+            uint32_t part[U];
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
+            for (int u = 0; u < U; ++u) {
                 sp[u] = miss[u] & spill_ok & (kw[u] != kEmpty) & inwin[u];
+                if constexpr (NUL) sp[u] = sp[u] & !vn[u] & !esc[u];
                 part[u] = (sp[u] && part_shift < 64) ? static_cast<uint32_t>(m[u] >> part_shift) & part_mask : 0u;
             }
 #pragma unroll
-            for (int u = 0; u < 2; ++u) pos[u] = sp[u] ? atoms_add(sfill + part[u] * 4u, 1u) : 0u;
+            for (int u = 0; u < U; ++u) pos[u] = sp[u] ? atoms_add(sfill + part[u] * 4u, 1u) : 0u;
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
+            for (int u = 0; u < U; ++u) {
                 if (sp[u] && pos[u] < cell_cap) {
                     spill_store(kw[u], v[u], part[u], pos[u]);
-                } else if (miss[u]) {
-                    global_row(kw[u], v[u]);
+                } else if (NUL ? (miss[u] && (!vn[u] || esc[u] || kw[u] == kEmpty)) : miss[u]) {
+                    global_row(kw[u], v[u], NUL && esc[u], NUL && vn[u]);
                 }
+            }
+            if constexpr (NUL) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) touch_queue(miss[u] & vn[u] & !esc[u] & (kw[u] != kEmpty), kw[u], lane);
             }
         }
     }
@@ -640,6 +677,15 @@ __device__ __forceinline__ KT kz_ring(const unsigned char* keys, const uint8_t* 
 // ---------------------------------------------------------------------------------------------
 constexpr int kListCap = 192;  // list entries per warp: fewer than 64 carried plus a tile's 128
 
+// The predicate interval test in the column's type.
+template <typename T>
+__device__ __forceinline__ bool pred_pass(const PredInterval& pi, T x) {
+    return ((x >= from_bits<T>(pi.lo)) & (x <= from_bits<T>(pi.hi))) != (pi.invert != 0);
+}
+__host__ __device__ __forceinline__ int pred_size(int32_t t) {
+    return (t == QDB_INT32 || t == QDB_FLOAT) ? 4 : ((t == QDB_INT64 || t == QDB_DOUBLE) ? 8 : 0);
+}
+
 // A key's C++ remainder by the call's modulus (the fused key % m variant).
 template <typename KT>
 __device__ __forceinline__ KT kmod_key(const AggArgs& a, KT k) {
@@ -656,10 +702,15 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
     constexpr bool VALS = (MODE & FM_VALS) != 0;
     constexpr bool KZ = !COMP && (MODE & FM_KZ) != 0;
     constexpr bool KMOD = !COMP && !KZ && (MODE & FM_KMOD) != 0 && std::is_integral<KT>::value;
+    constexpr bool NUL = !COMP && (MODE & FM_NULL) != 0;
+    constexpr bool WIDE = (MODE & FM_WIDE) != 0;
+    constexpr bool LIST = HAS_PRED || NUL;  // rows are filtered into the warp's list
+    // Rows a lane takes per step: a warp's whole slice of a tile where every row passes, two where they come off the list.
+    constexpr int U = LIST ? 2 : kFastSeg;
     using PL = typename std::conditional<HAS_PRED, PT, int32_t>::type;
     constexpr int PW = sizeof(PL);
 
-    const FTab tab = ftab(sm, a);
+    const FTab tab = ftab<VT>(sm, a);
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(sm + a.so_bar);
     uint64_t* empty_bar = full_bar + a.NS;
     const int warp = threadIdx.x >> 5;
@@ -670,7 +721,7 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
     unsigned char* ring = sm + a.so_stage;
     const StageLayout& sl = a.sl;
 
-    ftab_init<VT>(sm, a, threadIdx.x, blockDim.x);
+    ftab_init<VT, WIDE>(sm, a, threadIdx.x, blockDim.x);
     if (spill_on) {
         for (int i = threadIdx.x; i < parts + kSeenWords; i += blockDim.x) sfill[i] = 0u;
         if (blockIdx.x == 0 && threadIdx.x == 0) a.spill_fill[static_cast<int64_t>(parts) * a.spill_ctas] = 0u;  // spill-pass work counter
@@ -702,6 +753,15 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
             uint32_t tx = static_cast<uint32_t>(kFastT) * sizeof(KT) * ((COMP ? 2 : 1) - (KZ ? 1 : 0));
             if (VALS) tx += static_cast<uint32_t>(kFastT) * sizeof(VT);
             if (HAS_PRED) tx += static_cast<uint32_t>(kFastT) * PW;
+            constexpr uint32_t NB8 = kFastT / 8;  // bytes of a tile's null words
+            const uint32_t rpw = NUL ? static_cast<uint32_t>(pred_size(a.ptype)) : 0u;
+            if constexpr (NUL) {
+                tx += static_cast<uint32_t>(kFastT) * rpw;
+                if (a.knull0) tx += NB8;
+                if (a.vnull) tx += NB8;
+                if (a.pnull) tx += NB8;
+                if (a.mask) tx += kFastT;
+            }
             for (; q < my_tiles; ++q) {
                 const int64_t tile = blockIdx.x + q * static_cast<int64_t>(gridDim.x);
                 if (tile >= a.full_tiles) break;  // the partial last tile is read directly
@@ -746,6 +806,15 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
                 if (COMP) bulk_g2s(ring + sl.key1 + so * sizeof(KT), static_cast<const KT*>(a.key1) + r0, kFastT * sizeof(KT), &full_bar[s], pol);
                 if (VALS) bulk_g2s(ring + sl.val + so * sizeof(VT), static_cast<const VT*>(a.vals) + r0, kFastT * sizeof(VT), &full_bar[s], pol);
                 if (HAS_PRED) bulk_g2s(ring + sl.pred + so * PW, static_cast<const PL*>(a.pcol) + r0, kFastT * PW, &full_bar[s], pol);
+                if constexpr (NUL) {
+                    const size_t sn = static_cast<size_t>(s) * NB8;
+                    const int64_t w0 = r0 / 64;
+                    if (rpw) bulk_g2s(ring + sl.pred + so * rpw, static_cast<const unsigned char*>(a.pcol) + r0 * rpw, kFastT * rpw, &full_bar[s], pol);
+                    if (a.knull0) bulk_g2s(ring + sl.knull0 + sn, a.knull0 + w0, NB8, &full_bar[s], pol);
+                    if (a.vnull) bulk_g2s(ring + sl.vnull + sn, a.vnull + w0, NB8, &full_bar[s], pol);
+                    if (a.pnull) bulk_g2s(ring + sl.pnull + sn, a.pnull + w0, NB8, &full_bar[s], pol);
+                    if (a.mask) bulk_g2s(ring + sl.mask + so, a.mask + r0, kFastT, &full_bar[s], pol);
+                }
                 if (++s == a.NS) {
                     s = 0;
                     ph ^= 1u;
@@ -780,22 +849,22 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
                 for (int j = lane; j < kFastR; j += 32) {
                     const int i = warp * kFastR + j;
                     const int64_t r = tile * kFastT + i;
-                    if (r < a.n) e = max(e, fexp<VT>(staged ? rv[i] : static_cast<const VT*>(a.vals)[r]));
+                    if (r < a.n && !(NUL && null_bit(a.vnull, r)))
+                        e = max(e, fexp<VT>(staged ? rv[i] : static_cast<const VT*>(a.vals)[r]));
                 }
             }
             e = __reduce_max_sync(0xffffffffu, e);
             if (lane == 0 && e != INT_MIN) atomicMax(&s_emax, e);
         }
         asm volatile("bar.sync 1, %0;" ::"r"(kFastWarps * 32) : "memory");
-        fq = fixq<VT>(s_emax == INT_MIN ? 0 : s_emax, hb);
+        fq = fixq<VT, WIDE>(s_emax == INT_MIN ? 0 : s_emax, hb);
 
         FastWarp<VT, MODE> fw(a, tab, fq, &s_claims);
         fw.bshift = 32;
         fw.fits = a.fits != 0;
+        fw.counting = !fw.fits;
         fw.probe_b = a.probe_b;
         fw.spill_ok = spill_on;
-        // Warp aggregation pays only when lanes often share a slot: tried on tables sized for every group.
-        fw.dedup = a.dedup == 1 || (a.dedup == 2 && a.fits != 0);
         if (spill_on) {
             fw.sfill = smem_u32(sfill);
             fw.seen = smem_u32(sfill + parts);
@@ -803,13 +872,34 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
             fw.part_shift = 64 - a.spill_bits;
             fw.part_mask = static_cast<uint32_t>(parts - 1);
             fw.cell_base = blockIdx.x;
-            fw.cell_mul = a.spill_ctas;
+            fw.cell_mul = static_cast<uint32_t>(a.spill_ctas);
             fw.spill_out = a.spill_keys;
         }
         auto pass = [&](PL x) -> bool { return ((x >= plo) & (x <= phi)) != pinv; };
+        if constexpr (NUL) fw.touch = reinterpret_cast<uint64_t*>(sm + a.so_touch) + warp * kTouchCap;
+        // Null bit of the staged row g (stage s, row i at g = s T + i).
+        auto ring_bit = [&](int32_t off, int g) -> bool {
+            return off >= 0 && ((reinterpret_cast<const uint32_t*>(ring + off)[g >> 5] >> (g & 31)) & 1u);
+        };
+        // FM_NULL's filter: the predicate in its own type, its NULLs and the row mask.
+        auto pass_any = [&](const void* col, int64_t i) -> bool {
+            switch (a.ptype) {
+                case QDB_INT32: return pred_pass<int32_t>(a.pi, static_cast<const int32_t*>(col)[i]);
+                case QDB_INT64: return pred_pass<int64_t>(a.pi, static_cast<const int64_t*>(col)[i]);
+                case QDB_FLOAT: return pred_pass<float>(a.pi, static_cast<const float*>(col)[i]);
+                case QDB_DOUBLE: return pred_pass<double>(a.pi, static_cast<const double*>(col)[i]);
+                default: return true;
+            }
+        };
         const uint8_t* kzb = reinterpret_cast<const uint8_t*>(sm + a.so_bar + 96);
-        auto ring_row = [&](int g, uint64_t& kw, VT& v) {
-            if constexpr (COMP) kw = composite_word(static_cast<int32_t>(rk0[g]), static_cast<int32_t>(rk1[g]));
+        auto ring_row = [&](int g, uint64_t& kw, VT& v, bool& vn, bool& esc) {
+            vn = esc = false;
+            if constexpr (NUL) {
+                const bool kn = ring_bit(sl.knull0, g);
+                kw = kn ? kNullWord : key_word(rk0[g]);
+                esc = !kn & (kw == kNullWord);
+                vn = ring_bit(sl.vnull, g);
+            } else if constexpr (COMP) kw = composite_word(static_cast<int32_t>(rk0[g]), static_cast<int32_t>(rk1[g]));
             else if constexpr (KZ) kw = key_word(kz_ring<KT>(ring + sl.key0, kzb, g, a.kz_off));
             else kw = key_word(rk0[g]);
             if constexpr (VALS) v = rv[g];
@@ -818,20 +908,20 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
         // Steps over list entries [e0, e1): full 64-row steps, and the remainder when `flush`.  Returns the entries taken.
         auto steps = [&](int total, bool flush) -> int {
             int e0 = 0;
-            for (; e0 + 64 <= total || (flush && e0 < total); e0 += 64) {
-                bool act[2];
-                uint64_t kw[2];
-                VT v[2];
+            for (; e0 + 32 * U <= total || (flush && e0 < total); e0 += 32 * U) {
+                bool act[U], vn[U], esc[U];
+                uint64_t kw[U];
+                VT v[U];
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
+                for (int u = 0; u < U; ++u) {
                     const int e = e0 + 32 * u + lane;
                     act[u] = e < total;
                     int g;
-                    if constexpr (HAS_PRED) g = list[act[u] ? e : e0];
+                    if constexpr (LIST) g = list[act[u] ? e : e0];
                     else g = list[0] + (act[u] ? e : e0);  // list[0]: the first row of the warp's slice
-                    ring_row(g, kw[u], v[u]);
+                    ring_row(g, kw[u], v[u], vn[u], esc[u]);
                 }
-                fw.rows2(act, kw, v, static_cast<unsigned>(lane));
+                fw.template rows<U>(act, kw, v, vn, esc, static_cast<unsigned>(lane));
             }
             return e0 < total ? e0 : total;
         };
@@ -853,7 +943,17 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
                 const KT* k1p = static_cast<const KT*>(a.key1) + base;
                 const VT* vp = static_cast<const VT*>(a.vals) + base;
                 int count = 0;
-                if constexpr (HAS_PRED) {
+                if constexpr (NUL) {
+#pragma unroll
+                    for (int j = 0; j < kFastSeg; ++j) {
+                        const int i = w0 + 32 * j + lane;
+                        const int64_t r = base + i;
+                        const bool keep = i < lim && !null_bit(a.pnull, r) && (!a.mask || a.mask[r]) && pass_any(a.pcol, r);
+                        const uint32_t bj = __ballot_sync(0xffffffffu, keep);
+                        if (keep) list[count + __popc(bj & lt_mask)] = static_cast<uint16_t>(i);
+                        count += __popc(bj);
+                    }
+                } else if constexpr (HAS_PRED) {
                     const PL* pp = static_cast<const PL*>(a.pcol) + base;
 #pragma unroll
                     for (int j = 0; j < kFastSeg; ++j) {
@@ -867,23 +967,28 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
                     count = static_cast<int>(lim - w0 < 0 ? 0 : (lim - w0 > kFastR ? kFastR : lim - w0));
                 }
                 __syncwarp();
-                for (int e0 = 0; e0 < count; e0 += 64) {
-                    bool act[2];
-                    uint64_t kw[2];
-                    VT v[2];
+                for (int e0 = 0; e0 < count; e0 += 32 * U) {
+                    bool act[U], vn[U] = {}, esc[U] = {};
+                    uint64_t kw[U];
+                    VT v[U];
 #pragma unroll
-                    for (int u = 0; u < 2; ++u) {
+                    for (int u = 0; u < U; ++u) {
                         const int e = e0 + 32 * u + lane;
                         act[u] = e < count;
-                        const int i = HAS_PRED ? list[act[u] ? e : e0] : w0 + (act[u] ? e : e0);
-                        if constexpr (COMP) kw[u] = composite_word(static_cast<int32_t>(k0p[i]), static_cast<int32_t>(k1p[i]));
+                        const int i = LIST ? list[act[u] ? e : e0] : w0 + (act[u] ? e : e0);
+                        if constexpr (NUL) {
+                            const bool kn = null_bit(a.knull0, base + i);
+                            kw[u] = kn ? kNullWord : key_word(k0p[i]);
+                            esc[u] = !kn & (kw[u] == kNullWord);
+                            vn[u] = null_bit(a.vnull, base + i);
+                        } else if constexpr (COMP) kw[u] = composite_word(static_cast<int32_t>(k0p[i]), static_cast<int32_t>(k1p[i]));
                         else if constexpr (KZ) kw[u] = key_word(kz_key<KT>(a, base + i));
                         else if constexpr (KMOD) kw[u] = key_word(kmod_key<KT>(a, k0p[i]));
                         else kw[u] = key_word(k0p[i]);
                         if constexpr (VALS) v[u] = vp[i];
                         else v[u] = VT{};
                     }
-                    fw.rows2(act, kw, v, static_cast<unsigned>(lane));
+                    fw.template rows<U>(act, kw, v, vn, esc, static_cast<unsigned>(lane));
                 }
                 __syncwarp();
                 continue;
@@ -909,7 +1014,16 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
             }
             int total = lc;
             if (!full) {
-                if constexpr (HAS_PRED) {
+                if constexpr (NUL) {
+#pragma unroll
+                    for (int j = 0; j < kFastSeg; ++j) {
+                        const int g = g0 + 32 * j + lane;
+                        const bool keep = !ring_bit(sl.pnull, g) && (sl.mask < 0 || ring[sl.mask + g]) && pass_any(ring + sl.pred, g);
+                        const uint32_t bj = __ballot_sync(0xffffffffu, keep);
+                        if (keep) list[total + __popc(bj & lt_mask)] = static_cast<uint16_t>(g);
+                        total += __popc(bj);
+                    }
+                } else if constexpr (HAS_PRED) {
                     // Filter: segment j of the warp's slice is rows 32 j + lane; its ballot lists the passing rows in
                     // row order behind the carried entries.
 #pragma unroll
@@ -953,13 +1067,17 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
             // groups than the table holds) it stops probing the table and sends every row to the spill, which the
             // spill pass aggregates partition by partition in shared memory.
             if (q + 1 == kCountTile) fw.hits = fw.tries = 0;
-            if (q == kDecideTile && fw.use_smem) {
+            if (q == kDecideTile && fw.use_smem && fw.counting) {
                 const unsigned h = __reduce_add_sync(0xffffffffu, fw.hits);
                 const unsigned t = __reduce_add_sync(0xffffffffu, fw.tries);
                 if (t >= 256 && h * 8u < t) fw.use_smem = false;
                 fw.counting = false;
             }
             __syncwarp();
+        }
+        if constexpr (NUL) {
+            if (fw.touched > 32) fw.touch_drain(static_cast<unsigned>(lane), 32);
+            if (fw.touched > 0) fw.touch_drain(static_cast<unsigned>(lane), fw.touched);
         }
         if (held >= 0) {  // a wait that gave up left rows behind: release the stage all the same
             __syncwarp();
@@ -968,8 +1086,8 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
     }
 
     __syncthreads();
-    fq = fixq<VT>(s_emax == INT_MIN ? 0 : s_emax, hb);  // the producer warp's threads merge slots too
-    ftab_flush<VT>(sm, a, fq, &s_claims);
+    fq = fixq<VT, WIDE>(s_emax == INT_MIN ? 0 : s_emax, hb);  // the producer warp's threads merge slots too
+    ftab_flush<VT, WIDE>(sm, a, fq, &s_claims);
     if (spill_on)
         for (int i = threadIdx.x; i < parts; i += blockDim.x)
             a.spill_fill[static_cast<int64_t>(i) * a.spill_ctas + blockIdx.x] = min(sfill[i], static_cast<unsigned>(a.spill_cell));
@@ -996,8 +1114,9 @@ __global__ void __launch_bounds__(kFSpillThreads, 1) gb_fspill_kernel(const AggA
     __shared__ int s_item;
     constexpr bool VFLOAT = std::is_floating_point<VT>::value;
     constexpr bool VALS = (MODE & FM_VALS) != 0;
+    constexpr bool WIDE = (MODE & FM_WIDE) != 0;
     constexpr int kWarps = kFSpillThreads / 32;
-    const FTab tab = ftab(sm, a);
+    const FTab tab = ftab<VT>(sm, a);
     const int parts = 1 << a.spill_bits;
     const int items = parts * slices;
     unsigned* work = a.spill_fill + static_cast<int64_t>(parts) * a.spill_ctas;  // zeroed by the aggregation pass
@@ -1017,7 +1136,7 @@ __global__ void __launch_bounds__(kFSpillThreads, 1) gb_fspill_kernel(const AggA
             pre[0] = 0;
         }
         for (int i = threadIdx.x; i < parts2; i += blockDim.x) fill2[i] = 0u;
-        ftab_init<VT>(sm, a, threadIdx.x, blockDim.x);
+        ftab_init<VT, WIDE>(sm, a, threadIdx.x, blockDim.x);
         __syncthreads();
         const int item = s_item;
         if (item >= items) break;
@@ -1096,26 +1215,25 @@ __global__ void __launch_bounds__(kFSpillThreads, 1) gb_fspill_kernel(const AggA
         }
         __syncthreads();
         const int hb = max(1, 64 - __clzll(static_cast<long long>(total)));
-        const FixQ fq = fixq<VT>(s_emax == INT_MIN ? 0 : s_emax, hb);
+        const FixQ fq = fixq<VT, WIDE>(s_emax == INT_MIN ? 0 : s_emax, hb);
         FastWarp<VT, MODE> fw(a, tab, fq, &s_claims);
         fw.bshift = 32 - a.spill_bits;
         fw.fits = a.fits != 0;
         fw.probe_b = a.probe_b;
-        fw.dedup = a.dedup != 0;
         if (level2) {
             fw.spill_ok = true;
             fw.sfill = smem_u32(fill2);
             fw.cell_cap = static_cast<unsigned>(a.spill2_cell);
             fw.part_shift = 64 - a.spill_bits - a.spill2_bits;
             fw.part_mask = static_cast<uint32_t>(parts2 - 1);
-            fw.cell_base = static_cast<int64_t>(p) * parts2;
+            fw.cell_base = static_cast<uint32_t>(p) * static_cast<uint32_t>(parts2);
             fw.cell_mul = 1;
             fw.spill_out = a.spill2_keys;
         }
         for (; r0 < r_end; r0 += 64) {
             const int n0 = r0 + 64;
             if (n0 < r_end) load(n0, nact, nkw, nv);
-            fw.rows2(act, kw, v, static_cast<unsigned>(lane));
+            fw.template rows<2>(act, kw, v, static_cast<unsigned>(lane));
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 act[u] = nact[u];
@@ -1126,7 +1244,7 @@ __global__ void __launch_bounds__(kFSpillThreads, 1) gb_fspill_kernel(const AggA
         __syncthreads();
         for (int i = threadIdx.x; i < parts2; i += blockDim.x)
             a.spill2_fill[static_cast<int64_t>(p) * parts2 + i] = min(fill2[i], static_cast<unsigned>(a.spill2_cell));
-        ftab_flush<VT>(sm, a, fq, &s_claims);
+        ftab_flush<VT, WIDE>(sm, a, fq, &s_claims);
         __syncthreads();
     }
     if (threadIdx.x == 0) publish_claims(a.counters, a.capacity, s_claims);
@@ -1198,6 +1316,35 @@ int32_t launch_fast_m(const AggArgs& a, size_t smem, cudaStream_t st) {
     }
 }
 
+// Calls with NULL masks or a row mask (single key): one instantiation per key type, value type and aggregate set.
+template <typename KT, typename VT, int MODE>
+int32_t launch_fast_nul_t(const AggArgs& a, size_t smem, cudaStream_t st) {
+    constexpr int W = (std::is_same<VT, double>::value && (MODE & FM_SUM)) ? FM_WIDE : 0;
+    return launch_fast_t<KT, false, VT, NoPred, MODE | FM_NULL | W>(a, smem, st);
+}
+
+template <typename KT, typename VT>
+int32_t launch_fast_nul_m(const AggArgs& a, size_t smem, cudaStream_t st) {
+    switch (fast_mode(a)) {
+        case FM_VALS | FM_SUM: return launch_fast_nul_t<KT, VT, FM_VALS | FM_SUM>(a, smem, st);
+        case FM_VALS | FM_MM: return launch_fast_nul_t<KT, VT, FM_VALS | FM_MM>(a, smem, st);
+        case FM_VALS | FM_SUM | FM_MM: return launch_fast_nul_t<KT, VT, FM_VALS | FM_SUM | FM_MM>(a, smem, st);
+        default: return fail(QDB_ERR_INVALID, "gb_fast_kernel: unsupported aggregate set");
+    }
+}
+
+template <typename KT>
+int32_t launch_fast_nul_k(const AggArgs& a, ValKind vk, size_t smem, cudaStream_t st) {
+    if (fast_mode(a) == 0) return launch_fast_nul_t<KT, int32_t, 0>(a, smem, st);
+    switch (vk) {
+        case VK_I32: return launch_fast_nul_m<KT, int32_t>(a, smem, st);
+        case VK_I64: return launch_fast_nul_m<KT, int64_t>(a, smem, st);
+        case VK_F32: return launch_fast_nul_m<KT, float>(a, smem, st);
+        case VK_F64: return launch_fast_nul_m<KT, double>(a, smem, st);
+        default: return fail(QDB_ERR_INVALID, "unsupported value type");
+    }
+}
+
 template <typename KT, bool COMP, typename PT, bool KM>
 int32_t launch_fast_v(const AggArgs& a, ValKind vk, size_t smem, cudaStream_t st) {
     if (fast_mode(a) == 0) return launch_fast_z<KT, COMP, int32_t, PT, 0, KM>(a, smem, st);
@@ -1224,6 +1371,12 @@ int32_t launch_fast_k(const AggArgs& a, ValKind vk, int32_t ptype, size_t smem, 
 
 template <typename VT>
 int32_t launch_fspill_m(const AggArgs& a, size_t smem, int64_t grid, int32_t slices, cudaStream_t st) {
+    if constexpr (std::is_same<VT, double>::value) {
+        if (a.wide && fast_mode(a) == (FM_VALS | FM_SUM))
+            return launch_fspill_t<VT, FM_VALS | FM_SUM | FM_WIDE>(a, smem, grid, slices, st);
+        if (a.wide && fast_mode(a) == (FM_VALS | FM_SUM | FM_MM))
+            return launch_fspill_t<VT, FM_VALS | FM_SUM | FM_MM | FM_WIDE>(a, smem, grid, slices, st);
+    }
     switch (fast_mode(a)) {
         case FM_VALS | FM_SUM: return launch_fspill_t<VT, FM_VALS | FM_SUM>(a, smem, grid, slices, st);
         case FM_VALS | FM_MM: return launch_fspill_t<VT, FM_VALS | FM_MM>(a, smem, grid, slices, st);
@@ -1239,6 +1392,10 @@ int32_t launch_fast_i32_mod(const AggArgs& a, ValKind vk, int32_t ptype, size_t 
 int32_t launch_fast_i64_mod(const AggArgs& a, ValKind vk, int32_t ptype, size_t smem, cudaStream_t st);
 int32_t launch_fast_f32(const AggArgs& a, ValKind vk, int32_t ptype, size_t smem, cudaStream_t st);
 int32_t launch_fast_f64(const AggArgs& a, ValKind vk, int32_t ptype, size_t smem, cudaStream_t st);
+int32_t launch_fast_i32_nul(const AggArgs& a, ValKind vk, size_t smem, cudaStream_t st);
+int32_t launch_fast_i64_nul(const AggArgs& a, ValKind vk, size_t smem, cudaStream_t st);
+int32_t launch_fast_f32_nul(const AggArgs& a, ValKind vk, size_t smem, cudaStream_t st);
+int32_t launch_fast_f64_nul(const AggArgs& a, ValKind vk, size_t smem, cudaStream_t st);
 int32_t launch_fast_comp(const AggArgs& a, ValKind vk, int32_t ptype, size_t smem, cudaStream_t st);
 
 }  // namespace qdb
