@@ -649,8 +649,7 @@ int32_t qdb_gb_max_hash_count(qdb_gb* gb, int64_t* out) {
 int32_t qdb_gb_group_count(qdb_gb* gb, int64_t* out, void* stream) {
     if (!gb || !out) return fail(QDB_ERR_INVALID, "qdb_gb_group_count: null argument");
     unsigned long long h = 0;
-    QDB_CUDA_TRY(cudaMemcpyAsync(&h, gb->counters, sizeof(h), cudaMemcpyDeviceToHost, as_stream(stream)));
-    QDB_CUDA_TRY(cudaStreamSynchronize(as_stream(stream)));
+    QDB_CUDA_TRY(read_back(&h, gb->counters, sizeof(h), as_stream(stream)));
     *out = static_cast<int64_t>(h);
     return QDB_OK;
 }
@@ -965,8 +964,7 @@ int32_t qdb_gb_check(qdb_gb* gb, void* stream) {
     if (!gb) return fail(QDB_ERR_INVALID, "qdb_gb_check: null table");
     cudaStream_t s = as_stream(stream);
     int32_t status = 0;
-    QDB_CUDA_TRY(cudaMemcpyAsync(&status, &gb->counters[1], sizeof(status), cudaMemcpyDeviceToHost, s));
-    QDB_CUDA_TRY(cudaStreamSynchronize(s));
+    QDB_CUDA_TRY(read_back(&status, &gb->counters[1], sizeof(status), s));
     if (status != QDB_OK) {
         QDB_CUDA_TRY(cudaMemsetAsync(&gb->counters[1], 0, sizeof(unsigned long long), s));
         if (status == QDB_HASH_TABLE_FULL)

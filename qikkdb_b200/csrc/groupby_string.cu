@@ -285,8 +285,7 @@ static int32_t gbs_build_keys(const GbsDict& t, const int32_t* slots, const uint
         gbs_len_kernel<<<gbs_grid(static_cast<uint64_t>(groups)), 256, 0, s>>>(t, slots, knull, groups, clen);
         note_launch();
         rc = exclusive_scan<long long>(clen, groups, tot, s);
-        cudaError_t e = rc == QDB_OK ? cudaMemcpyAsync(&nchars, tot, 8, cudaMemcpyDeviceToHost, s) : cudaSuccess;
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        const cudaError_t e = rc == QDB_OK ? read_back(&nchars, tot, 8, s) : cudaSuccess;
         if (rc == QDB_OK && e != cudaSuccess) rc = cuda_fail(e, "string keys: lengths");
     }
     if (rc == QDB_OK)
@@ -422,8 +421,7 @@ int32_t qdb_gbs_process(qdb_gbs* g, const char* chars, const int64_t* ends, cons
 int32_t qdb_gbs_check(qdb_gbs* g, void* stream) {
     if (!g) return fail(QDB_ERR_INVALID, "qdb_gbs_check: null table");
     unsigned long long st = 0;
-    QDB_CUDA_TRY(cudaMemcpyAsync(&st, g->t.counters + 1, 8, cudaMemcpyDeviceToHost, as_stream(stream)));
-    QDB_CUDA_TRY(cudaStreamSynchronize(as_stream(stream)));
+    QDB_CUDA_TRY(read_back(&st, g->t.counters + 1, 8, as_stream(stream)));
     const int32_t status = static_cast<int32_t>(st & 0xffffffffu);
     if (status != QDB_OK) {
         QDB_CUDA_TRY(cudaMemsetAsync(g->t.counters + 1, 0, 8, as_stream(stream)));

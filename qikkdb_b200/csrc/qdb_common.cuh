@@ -42,6 +42,10 @@ void note_launch(int64_t n = 1);
 int32_t dev_alloc(void** p, size_t bytes, cudaStream_t s);
 void dev_free(void* p, cudaStream_t s);
 
+// Copies `bytes` (at most 64) from the device on stream s and waits for them, through page-locked memory of the calling
+// thread (a copy into pageable memory goes through a staging buffer of the driver: about 4 us more).
+cudaError_t read_back(void* dst, const void* src, size_t bytes, cudaStream_t s);
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 inline int type_size(int32_t t) {

@@ -190,8 +190,7 @@ static int32_t count_and_scan(const int8_t* mask, int64_t n, bool sum_values, lo
     rc_scan_kernel<<<1, kRcThreads, 0, s>>>(*offsets, ntiles);
     note_launch();
     if (total) {
-        cudaError_t e = cudaMemcpyAsync(total, *offsets + ntiles, sizeof(long long), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        const cudaError_t e = read_back(total, *offsets + ntiles, sizeof(long long), s);
         if (e != cudaSuccess) {
             dev_free(*offsets, s);
             *offsets = nullptr;

@@ -48,7 +48,8 @@ __device__ __forceinline__ int block_excl_scan(int x, int* total) {
 // chunk start + w kResWarpSlots, 32 at a time (one slot per lane), so every load of the key words is coalesced.
 constexpr int kResWarpSlots = kResChunk / (kResThreads / 32);
 
-__global__ void res_count_kernel(SlotSpace sp, int* chunk_counts) {
+// A table of one chunk needs no scan: its offset is 0 and its count the total.
+__global__ void res_count_kernel(SlotSpace sp, int* chunk_counts, long long* total_out) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint64_t wbase = static_cast<uint64_t>(blockIdx.x) * kResChunk + static_cast<uint64_t>(warp) * kResWarpSlots;
     int c = 0;
@@ -56,7 +57,10 @@ __global__ void res_count_kernel(SlotSpace sp, int* chunk_counts) {
     for (int i = 0; i < kResWarpSlots; i += 32) c += present(sp, wbase + i + lane) ? 1 : 0;
     __shared__ int tot;
     block_excl_scan(c, &tot);
-    if (threadIdx.x == 0) chunk_counts[blockIdx.x] = tot;
+    if (threadIdx.x == 0) {
+        chunk_counts[blockIdx.x] = gridDim.x == 1 ? 0 : tot;
+        if (gridDim.x == 1) *total_out = tot;
+    }
 }
 
 // Exclusive scan of the chunk counts in one block; total written to counts[nchunks].
@@ -301,29 +305,23 @@ int32_t qdb_gb_results_multi(qdb_gb* gb, int32_t n_aggs, const int32_t* aggs, vo
     const SlotSpace sp = slot_space(gb);
     const int64_t nchunks = static_cast<int64_t>((sp.total + kResChunk - 1) / kResChunk);
 
-    int* counts = nullptr;
-    long long* d_total = nullptr;
-    int32_t rc = dev_alloc(reinterpret_cast<void**>(&counts), (nchunks + 1) * sizeof(int), s);
+    long long* d_total = nullptr;  // the group count, then the chunk counts
+    int32_t rc = dev_alloc(reinterpret_cast<void**>(&d_total), sizeof(long long) + (nchunks + 1) * sizeof(int), s);
     if (rc != QDB_OK) return rc;
-    rc = dev_alloc(reinterpret_cast<void**>(&d_total), sizeof(long long), s);
-    if (rc != QDB_OK) {
-        dev_free(counts, s);
-        return rc;
+    int* counts = reinterpret_cast<int*>(d_total + 1);
+    res_count_kernel<<<static_cast<unsigned>(nchunks), kResThreads, 0, s>>>(sp, counts, d_total);
+    note_launch();
+    if (nchunks > 1) {
+        res_scan_kernel<<<1, kResThreads, 0, s>>>(counts, nchunks, d_total);
+        note_launch();
     }
-    res_count_kernel<<<static_cast<unsigned>(nchunks), kResThreads, 0, s>>>(sp, counts);
-    note_launch();
-    res_scan_kernel<<<1, kResThreads, 0, s>>>(counts, nchunks, d_total);
-    note_launch();
     long long total = 0;
-    cudaError_t e = cudaMemcpyAsync(&total, d_total, sizeof(total), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaError_t e = read_back(&total, d_total, sizeof(total), s);
     if (e != cudaSuccess) {
-        dev_free(counts, s);
         dev_free(d_total, s);
         return cuda_fail(e, "qdb_gb_results: count pass");
     }
     if (total == 0) {
-        dev_free(counts, s);
         dev_free(d_total, s);
         return QDB_OK;
     }
@@ -364,7 +362,6 @@ int32_t qdb_gb_results_multi(qdb_gb* gb, int32_t n_aggs, const int32_t* aggs, vo
             out_vals[i] = nullptr;
             if (out_val_nulls) out_val_nulls[i] = nullptr;
         }
-        dev_free(counts, s);
         dev_free(d_total, s);
         return rc;
     }
@@ -380,7 +377,6 @@ int32_t qdb_gb_results_multi(qdb_gb* gb, int32_t n_aggs, const int32_t* aggs, vo
     res_emit_kernel<<<static_cast<unsigned>(nchunks), kResThreads, 0, s>>>(ea);
     note_launch();
     e = cudaGetLastError();
-    dev_free(counts, s);
     dev_free(d_total, s);
     if (e != cudaSuccess) return cuda_fail(e, "res_emit_kernel");
     *out_count = total;

@@ -70,6 +70,30 @@ int32_t dev_alloc(void** p, size_t bytes, cudaStream_t s) {
     return QDB_OK;
 }
 
+namespace {
+struct HostWords {  // 64 bytes per thread, given back when the thread ends
+    void* p = nullptr;
+    HostWords() {
+        if (cudaHostAlloc(&p, 64, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+    }
+    ~HostWords() {
+        if (p) cudaFreeHost(p);
+    }
+};
+}  // namespace
+
+cudaError_t read_back(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    static thread_local HostWords words;
+    void* to = (words.p && bytes <= 64) ? words.p : dst;
+    cudaError_t e = cudaMemcpyAsync(to, src, bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && to != dst) memcpy(dst, to, bytes);
+    return e;
+}
+
 void dev_free(void* p, cudaStream_t s) {
     if (p) cudaFreeAsync(p, s);
 }

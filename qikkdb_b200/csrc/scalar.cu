@@ -312,8 +312,7 @@ int32_t qdb_scalar_process(qdb_scalar* q, const void* vals, const uint64_t* val_
 int32_t qdb_scalar_result(qdb_scalar* q, int32_t agg, void* out_value, int32_t* out_is_null, void* stream) {
     if (!q || !out_value) return fail(QDB_ERR_INVALID, "qdb_scalar_result: bad arguments");
     ScalarState h{};
-    QDB_CUDA_TRY(cudaMemcpyAsync(&h, q->st, sizeof(h), cudaMemcpyDeviceToHost, as_stream(stream)));
-    QDB_CUDA_TRY(cudaStreamSynchronize(as_stream(stream)));
+    QDB_CUDA_TRY(read_back(&h, q->st, sizeof(h), as_stream(stream)));
     const bool empty = h.count == 0;
     if (out_is_null) *out_is_null = (agg != QDB_AGG_COUNT && empty) ? 1 : 0;
     if (agg == QDB_AGG_COUNT) {
