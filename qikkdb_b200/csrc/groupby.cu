@@ -399,8 +399,8 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
         }
     sl.bytes = stage_bytes;
 
-    const bool has_mm = a.has_min || a.has_max;
-    const size_t slot_bytes = 8 + 4 + (a.has_sum ? (a.wide ? 12 : 8) : 0) + (has_mm ? (vk_is_32(vk) ? 8 : 16) : 0);
+    const size_t mm_bytes = vk_is_32(vk) ? 4 : 8;  // of one encoded minimum or maximum
+    const size_t slot_bytes = 8 + 4 + (a.has_sum ? (a.wide ? 12 : 8) : 0) + (a.has_min ? mm_bytes : 0) + (a.has_max ? mm_bytes : 0);
     const size_t bucket_bytes = 2 * slot_bytes;
     auto layout_table = [&](AggArgs& x, int NB, int rep) {  // offsets of the table arrays; returns the bytes used
         const size_t S = static_cast<size_t>(NB) * 2;
@@ -409,7 +409,8 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
         x.NB = NB;
         x.rep_shift = rep;
         x.so_keys = static_cast<int32_t>(o); o += S * 8;
-        x.so_mn = static_cast<int32_t>(o); o += has_mm ? E * (vk_is_32(vk) ? 8 : 16) : 0;
+        x.so_mn = static_cast<int32_t>(o); o += a.has_min ? E * mm_bytes : 0;
+        x.so_mx = static_cast<int32_t>(o); o += a.has_max ? E * mm_bytes : 0;
         x.so_cnt = static_cast<int32_t>(o); o += E * 4;
         x.so_l0 = static_cast<int32_t>(o); o += a.has_sum ? E * 4 : 0;
         x.so_l1 = static_cast<int32_t>(o); o += a.has_sum ? E * 4 : 0;
@@ -447,7 +448,7 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
                                prefix2 - fill2_bytes;
         NB2 = static_cast<int>(budget2 / bucket_bytes);
         if (NB2 >= 64 && env_int("QDB_AGG_NO_SPILL", 0) == 0) {
-            const uint64_t per = static_cast<uint64_t>(NB2);  // distinct keys per partition at half load
+            const uint64_t per = static_cast<uint64_t>(NB2) + NB2 / 8;  // distinct keys per partition at 9/16 load
             // At least two partitions per SM (512 on 148 SMs), so the spill pass's items balance over the SMs (the
             // last wave of a pass with 1.7 items per SM leaves a quarter of them idle); more partitions measured
             // slower (2^28-row filtered workload, aggregation + spill: 2.27 / 2.31 / 2.58 / 3.02 ms at 2 / 4 / 8 / 16

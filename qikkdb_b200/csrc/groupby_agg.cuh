@@ -107,6 +107,7 @@ struct AggArgs {
     int32_t null_keys = 0;
     int32_t wide = 0;
     int32_t so_touch = 0;
+    int32_t so_mx = 0;       // fast pass: maxima (minima at so_mn; each only when the table has the aggregate)
     int32_t rep_shift = 0; // 2^rep_shift copies of every slot's state (tables of few groups)
     int32_t pred_float = 0;  // the fast pass compares IEEE predicate values as order-preserving integers
     int32_t flush_rounds = 16;  // lock-step probe rounds of a shared table's merge into the global table

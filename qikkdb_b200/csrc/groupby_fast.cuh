@@ -48,6 +48,9 @@ __device__ __forceinline__ uint32_t atoms_or(uint32_t a, uint32_t x) {
     asm volatile("atom.shared.or.b32 %0, [%1], %2;" : "=r"(old) : "r"(a), "r"(x) : "memory");
     return old;
 }
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t x) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(x) : "memory");
+}
 __device__ __forceinline__ void lds128(uint32_t a, uint64_t& k0, uint64_t& k1) {
     asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(k0), "=l"(k1) : "r"(a) : "memory");
 }
@@ -59,7 +62,7 @@ __device__ __forceinline__ void lds128(uint32_t a, uint64_t& k0, uint64_t& k1) {
 // A table of few groups keeps 2^rep_shift copies of every state (slot s, copy r at index (s << rep_shift) + r); lane l
 // of every warp updates copy l mod 2^rep_shift and the merge adds the copies up.
 struct FTab {
-    uint32_t keys, cnt, l0, l1, l2, mm;  // state arrays: the address of this lane's copy of slot 0
+    uint32_t keys, cnt, l0, l1, l2, mn, mx;  // state arrays: the address of this lane's copy of slot 0
     uint32_t NB;
     uint32_t osh;                    // slot s's 4-byte state is at s << osh
 };
@@ -73,7 +76,8 @@ __device__ __forceinline__ FTab ftab(unsigned char* sm, const AggArgs& a) {
     t.l0 = smem_u32(sm + a.so_l0) + r * 4u;
     t.l1 = smem_u32(sm + a.so_l1) + r * 4u;
     t.l2 = smem_u32(sm + a.so_l2) + r * 4u;
-    t.mm = smem_u32(sm + a.so_mn) + r * (sizeof(VT) == 4 ? 8u : 16u);
+    t.mn = smem_u32(sm + a.so_mn) + r * static_cast<uint32_t>(sizeof(VT));
+    t.mx = smem_u32(sm + a.so_mx) + r * static_cast<uint32_t>(sizeof(VT));
     t.NB = static_cast<uint32_t>(a.NB);
     t.osh = 2u + static_cast<uint32_t>(a.rep_shift);
     return t;
@@ -208,8 +212,9 @@ __device__ __forceinline__ void ftab_init(unsigned char* sm, const AggArgs& a, i
     unsigned* cnt = reinterpret_cast<unsigned*>(sm + a.so_cnt);
     unsigned* l0 = reinterpret_cast<unsigned*>(sm + a.so_l0);
     unsigned* l1 = reinterpret_cast<unsigned*>(sm + a.so_l1);
-    unsigned long long* mm = reinterpret_cast<unsigned long long*>(sm + a.so_mn);
-    const bool has_mm = a.has_min || a.has_max;
+    using MT = typename std::conditional<sizeof(VT) == 4, int, long long>::type;  // encoded min / max
+    MT* mn = reinterpret_cast<MT*>(sm + a.so_mn);
+    MT* mx = reinterpret_cast<MT*>(sm + a.so_mx);
     for (int i = tid; i < S; i += nthreads) keys[i] = kEmpty;
     const int E = S << a.rep_shift;
     for (int i = tid; i < E; i += nthreads) {
@@ -219,14 +224,8 @@ __device__ __forceinline__ void ftab_init(unsigned char* sm, const AggArgs& a, i
             l1[i] = 0u;
             if (WIDE) reinterpret_cast<unsigned*>(sm + a.so_l2)[i] = 0u;
         }
-        if (has_mm) {
-            if (sizeof(VT) == 4) {
-                mm[i] = kPackedMinMaxInit;
-            } else {
-                mm[2 * i] = kMinInit64;
-                mm[2 * i + 1] = kMaxInit64;
-            }
-        }
+        if (a.has_min) mn[i] = sizeof(VT) == 4 ? static_cast<MT>(INT_MAX) : static_cast<MT>(kMinInit64);
+        if (a.has_max) mx[i] = sizeof(VT) == 4 ? static_cast<MT>(INT_MIN) : static_cast<MT>(kMaxInit64);
     }
 }
 
@@ -238,7 +237,7 @@ __device__ __forceinline__ void ftab_init(unsigned char* sm, const AggArgs& a, i
 
 template <typename VT, bool WIDE>
 __device__ __forceinline__ void ftab_flush(unsigned char* sm, const AggArgs& a, const FixQ& fq,
-                                           unsigned long long* claims) {
+                                           unsigned long long* claims, bool null_seen = true) {
     constexpr bool V32 = sizeof(VT) == 4;
     constexpr bool VFLOAT = std::is_floating_point<VT>::value;
     const int S = a.NB * 2;
@@ -248,7 +247,9 @@ __device__ __forceinline__ void ftab_flush(unsigned char* sm, const AggArgs& a, 
     const unsigned* l0 = reinterpret_cast<const unsigned*>(sm + a.so_l0);
     const unsigned* l1 = reinterpret_cast<const unsigned*>(sm + a.so_l1);
     const unsigned* l2 = reinterpret_cast<const unsigned*>(sm + a.so_l2);
-    const unsigned char* mm = sm + a.so_mn;
+    using MT = typename std::conditional<V32, int, long long>::type;
+    const MT* smn = reinterpret_cast<const MT*>(sm + a.so_mn);
+    const MT* smx = reinterpret_cast<const MT*>(sm + a.so_mx);
     const uint64_t mask = a.main.mask;
     constexpr int U = 4;
     for (int i0 = threadIdx.x; i0 < S; i0 += U * blockDim.x) {
@@ -262,7 +263,7 @@ __device__ __forceinline__ void ftab_flush(unsigned char* sm, const AggArgs& a, 
             g[u] = nullptr;
             pend[u] = key[u] != kEmpty;
             if (a.null_keys && key[u] == kNullWord) {
-                g[u] = g_special(a.main, W, 0, claims);
+                g[u] = null_seen ? g_special(a.main, W, 0, claims) : nullptr;
                 pend[u] = false;
             }
             pos[u] = pend[u] ? home_slot(a.main, mix64(key[u])) : 0ull;
@@ -314,17 +315,8 @@ __device__ __forceinline__ void ftab_flush(unsigned char* sm, const AggArgs& a, 
                     if (WIDE) wide += (static_cast<__int128>(static_cast<int32_t>(l2[e])) << 64) + static_cast<__int128>(lo);
                     else sum += lo;
                 }
-                if (a.has_min || a.has_max) {
-                    if (V32) {
-                        const int* w = reinterpret_cast<const int*>(mm) + 2 * e;
-                        mn = min(mn, static_cast<long long>(w[0]));
-                        mx = max(mx, static_cast<long long>(w[1]));
-                    } else {
-                        const long long* w = reinterpret_cast<const long long*>(mm) + 2 * e;
-                        mn = min(mn, w[0]);
-                        mx = max(mx, w[1]);
-                    }
-                }
+                if (a.has_min) mn = min(mn, static_cast<long long>(smn[e]));
+                if (a.has_max) mx = max(mx, static_cast<long long>(smx[e]));
             }
             uint64_t sumbits = sum;
             if (a.has_sum && VFLOAT) {
@@ -380,6 +372,9 @@ struct FastWarp {
     uint32_t cell_base = 0;
     uint32_t cell_mul = 0;
     uint64_t* spill_out = nullptr;
+    // The NULL key's slot, claimed before the first row (FM_NULL with NULL keys), and the word that a NULL key sets.
+    int null_slot = -1;
+    uint32_t null_seen = 0;
     // Keys of rows with a NULL value that missed the table (they only have to exist in the global table), looked up 32
     // at a time.
     uint64_t* touch = nullptr;
@@ -437,15 +432,12 @@ struct FastWarp {
         if constexpr (MM) {
             if constexpr (sizeof(VT) == 4) {
                 const int32_t e = enc32(v);
-                const uint32_t w = t.mm + o * 2u;
-                const uint64_t cur = lds64(w);
-                if (a.has_min && e < static_cast<int32_t>(cur)) reds_min32(w, e);
-                if (a.has_max && e > static_cast<int32_t>(cur >> 32)) reds_max32(w + 4u, e);
+                if (a.has_min && e < lds32(t.mn + o)) reds_min32(t.mn + o, e);
+                if (a.has_max && e > lds32(t.mx + o)) reds_max32(t.mx + o, e);
             } else {
                 const long long e = enc64(v);
-                const uint32_t w = t.mm + o * 4u;
-                if (a.has_min && e < lds64s(w)) reds_min64(w, e);
-                if (a.has_max && e > lds64s(w + 8u)) reds_max64(w + 8u, e);
+                if (a.has_min && e < lds64s(t.mn + o * 2u)) reds_min64(t.mn + o * 2u, e);
+                if (a.has_max && e > lds64s(t.mx + o * 2u)) reds_max64(t.mx + o * 2u, e);
             }
         }
     }
@@ -488,7 +480,7 @@ struct FastWarp {
             if constexpr (NUL) inwin[u] = inwin[u] | vn[u];
             m[u] = fhash(kw[u]);
             look[u] = act[u] & (kw[u] != kEmpty) & inwin[u] & use_smem;
-            if constexpr (NUL) look[u] = look[u] & !esc[u];
+            if constexpr (NUL) look[u] = look[u] & (kw[u] != kNullWord);
             b[u] = fbucket(m[u], bshift, t.NB);
             k0[u] = k1[u] = kEmpty;
         }
@@ -501,6 +493,14 @@ struct FastWarp {
             hit[u] = look[u] & (h0 | (k1[u] == kw[u]));
             slot[u] = hit[u] ? static_cast<int>(h0 ? b[u] : t.NB + b[u]) : -1;
             empty[u] = (k0[u] == kEmpty) | (k1[u] == kEmpty);
+            if constexpr (NUL) {
+                // NULL keys never leave the table, also when it is not probed: they may be a large share of the rows.
+                if (act[u] & (kw[u] == kNullWord) & !esc[u] & inwin[u]) {
+                    slot[u] = null_slot;
+                    hit[u] = true;
+                    if (lds32(null_seen) == 0) sts32(null_seen, 1u);
+                }
+            }
         }
         if (fits) {
             // A table sized for every group places a key whose home bucket is full in its second bucket, or rarely in one
@@ -697,6 +697,8 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ unsigned long long s_claims;
     __shared__ int s_emax;
+    __shared__ int s_null_slot;
+    __shared__ unsigned s_null_seen;
     constexpr bool HAS_PRED = !std::is_same<PT, NoPred>::value;
     constexpr bool VFLOAT = std::is_floating_point<VT>::value;
     constexpr bool VALS = (MODE & FM_VALS) != 0;
@@ -729,6 +731,8 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
     if (threadIdx.x == 0) {
         s_claims = 0;
         s_emax = INT_MIN;
+        s_null_slot = -1;
+        s_null_seen = 0u;
         for (int s = 0; s < a.NS; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], kFastWarps);
@@ -736,6 +740,11 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
         mbar_fence_init();
     }
     __syncthreads();
+    if constexpr (NUL) {
+        if (a.null_keys && threadIdx.x == 0)  // an empty table always has room in the home bucket
+            s_null_slot = fclaim(tab, fbucket(fhash(kNullWord), 32, tab.NB), kNullWord, 1);
+        __syncthreads();
+    }
 
     const int64_t my_tiles =
         (a.tiles > static_cast<int64_t>(blockIdx.x)) ? (a.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
@@ -876,6 +885,10 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
             fw.spill_out = a.spill_keys;
         }
         auto pass = [&](PL x) -> bool { return ((x >= plo) & (x <= phi)) != pinv; };
+        if constexpr (NUL) {
+            fw.null_slot = s_null_slot;
+            fw.null_seen = smem_u32(&s_null_seen);
+        }
         if constexpr (NUL) fw.touch = reinterpret_cast<uint64_t*>(sm + a.so_touch) + warp * kTouchCap;
         // Null bit of the staged row g (stage s, row i at g = s T + i).
         auto ring_bit = [&](int32_t off, int g) -> bool {
@@ -906,7 +919,8 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
             else v = VT{};
         };
         // Steps over list entries [e0, e1): full 64-row steps, and the remainder when `flush`.  Returns the entries taken.
-        auto steps = [&](int total, bool flush) -> int {
+        const bool listed = LIST && (HAS_PRED || a.ptype || a.mask || a.pnull);  // FM_NULL without a filter: every row passes
+        auto steps = [&](int total, bool flush, int g0) -> int {
             int e0 = 0;
             for (; e0 + 32 * U <= total || (flush && e0 < total); e0 += 32 * U) {
                 bool act[U], vn[U], esc[U];
@@ -917,8 +931,8 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
                     const int e = e0 + 32 * u + lane;
                     act[u] = e < total;
                     int g;
-                    if constexpr (LIST) g = list[act[u] ? e : e0];
-                    else g = list[0] + (act[u] ? e : e0);  // list[0]: the first row of the warp's slice
+                    if (listed) g = list[act[u] ? e : e0];
+                    else g = g0 + (act[u] ? e : e0);
                     ring_row(g, kw[u], v[u], vn[u], esc[u]);
                 }
                 fw.template rows<U>(act, kw, v, vn, esc, static_cast<unsigned>(lane));
@@ -1014,7 +1028,9 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
             }
             int total = lc;
             if (!full) {
-                if constexpr (NUL) {
+                if (NUL && !listed) {
+                    total = kFastR;
+                } else if constexpr (NUL) {
 #pragma unroll
                     for (int j = 0; j < kFastSeg; ++j) {
                         const int g = g0 + 32 * j + lane;
@@ -1035,13 +1051,12 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
                         total += __popc(bj);
                     }
                 } else {
-                    if (lane == 0) list[0] = static_cast<uint16_t>(g0);
                     total = kFastR;
                 }
                 __syncwarp();
             }
-            int taken = full ? total : steps(total, !keep_going);
-            if (held >= 0 && taken == 0) taken = steps(total, true);  // never hold two stages into the next tile
+            int taken = full ? total : steps(total, !keep_going, g0);
+            if (held >= 0 && taken == 0) taken = steps(total, true, g0);  // never hold two stages into the next tile
             __syncwarp();
             if (held >= 0 && lane == 0) mbar_arrive(&empty_bar[held]);  // its rows were the first lc entries
             held = -1;
@@ -1087,7 +1102,7 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
 
     __syncthreads();
     fq = fixq<VT, WIDE>(s_emax == INT_MIN ? 0 : s_emax, hb);  // the producer warp's threads merge slots too
-    ftab_flush<VT, WIDE>(sm, a, fq, &s_claims);
+    ftab_flush<VT, WIDE>(sm, a, fq, &s_claims, s_null_seen != 0u);
     if (spill_on)
         for (int i = threadIdx.x; i < parts; i += blockDim.x)
             a.spill_fill[static_cast<int64_t>(i) * a.spill_ctas + blockIdx.x] = min(sfill[i], static_cast<unsigned>(a.spill_cell));
