@@ -1,0 +1,8 @@
+// Aggregation pass of tables that hold every group (groupby_few.cuh), double keys.
+#include "groupby_few.cuh"
+
+namespace qdb {
+int32_t launch_few_f64(const AggArgs& a, ValKind vk, size_t smem, int64_t grid, cudaStream_t st) {
+    return launch_few_k<double, false>(a, vk, smem, grid, st);
+}
+}  // namespace qdb

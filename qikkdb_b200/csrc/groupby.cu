@@ -123,6 +123,18 @@ static int32_t launch_fast(const qdb_gb* gb, const AggArgs& a, int32_t ptype, si
     }
 }
 
+static int32_t launch_few(const qdb_gb* gb, const AggArgs& a, size_t smem, int64_t grid, cudaStream_t st) {
+    const ValKind vk = val_kind(gb->val_type);
+    if (gb->n_key_cols == 2) return launch_few_comp(a, vk, smem, grid, st);
+    switch (gb->key_type) {
+        case QDB_INT32: return launch_few_i32(a, vk, smem, grid, st);
+        case QDB_INT64: return launch_few_i64(a, vk, smem, grid, st);
+        case QDB_FLOAT: return launch_few_f32(a, vk, smem, grid, st);
+        case QDB_DOUBLE: return launch_few_f64(a, vk, smem, grid, st);
+        default: return fail(QDB_ERR_INVALID, "unsupported key type");
+    }
+}
+
 static int32_t launch_fspill(const qdb_gb* gb, const AggArgs& a, size_t smem, int64_t grid, int32_t slices,
                              cudaStream_t st) {
     if (fast_mode(a) == 0) return launch_fspill_t<int32_t, 0>(a, smem, grid, slices, st);
@@ -342,6 +354,7 @@ PredInterval pred_interval(const qdb_pred& p) {
 // columns are 16-byte aligned and hold at least one whole tile.  *used is false when the plan does not fit shared
 // memory (the caller then takes the general pass).
 // ---------------------------------------------------------------------------------------------
+constexpr int64_t kFewRows = 3072;     // rows of one step of a CTA of the pass without a ring (groupby_few.cuh: 768 x 4)
 constexpr size_t kMaxStates = 8192;  // states of a table with copies (clearing and merging them stays a few us)
 
 static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t ptype, cudaStream_t s, bool* used) {
@@ -428,6 +441,27 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
             ++rep;
         return rep;
     };
+
+    // A table that holds every group at half load or less (a quarter when it can) takes the pass without a ring, where the
+    // whole of shared memory is the table: a CTA per SM, or as many as there are steps of rows.
+    if (!a.nul && !a.kz) {
+        const size_t bytes = static_cast<size_t>(di.max_smem_optin) - 1024;
+        const uint64_t groups = static_cast<uint64_t>(gb->capacity) + 1;
+        uint64_t most = bytes / bucket_bytes;
+        const int64_t forced = env_int("QDB_FAST_BUCKETS", 0);
+        if (forced > 0) most = std::min<uint64_t>(most, static_cast<uint64_t>(forced));
+        if (groups <= most) {
+            const int NB = static_cast<int>(std::max<uint64_t>(16, std::min<uint64_t>(most, 2 * groups)));
+            const int64_t grid = std::min<int64_t>(di.sm_count, (a.n + kFewRows - 1) / kFewRows);
+            const size_t smem = layout_table(a, NB, rep_of(NB, a.n / grid, bytes));
+            a.fits = 1;
+            a.probe_b = std::min(kProbeBuckets, NB);
+            a.flush_rounds = static_cast<int32_t>(env_int("QDB_FLUSH_ROUNDS", 16));
+            a.ptype = ptype;
+            *used = true;
+            return launch_few(gb, a, smem, grid, s);
+        }
+    }
 
     // Spill plan: partitions small enough for the spill pass's table (one CTA per SM, the largest table shared
     // memory holds after the cell-fill prefix and the second-level counters) at half load.  The aggregation pass

@@ -8,9 +8,7 @@
 // consumer warps take the stages in order.  Warp w owns rows [128 w, 128 (w + 1)) of a tile and reads them as four
 // 32-row segments (lane l: rows 32 j + l), so the predicate loads are conflict-free and the ballot of segment j lists
 // its passing rows in row order.  The passing rows are then processed 32 at a time:
-//   * the key's bucket (four slots) holds four 15-bit tags in one 64-bit word: one 8-byte shared load and a
-//     zero-halfword test find the slot whose tag matches, one more load confirms the key; a key absent from a full
-//     bucket is a miss after that single load;
+//   * the key's bucket is two slots whose key words are read with one 16-byte load;
 //   * a hit updates the slot with 32-bit shared atomics only: a u32 count, a 64-bit sum kept as two u32 limbs (the
 //     carry out of the low limb is read from the value the atomic returns) and min/max issued only when the value
 //     improves on the slot's bound.  Integer sums wrap like the reference's 64-bit atomicAdd; float and double
@@ -343,7 +341,8 @@ constexpr int FM_NULL = 32;  // NULL masks (key, value, predicate) or a row mask
 constexpr int FM_WIDE = 64;  // 96-bit sums of doubles
 constexpr int FM_KMOD = 16;  // keys are replaced by key % m as they are read (single INT32 or INT64 key)
 
-template <typename VT, int MODE>
+// K32: every key word is a 32-bit key's, so none equals kEmpty.
+template <typename VT, int MODE, bool K32 = false>
 struct FastWarp {
     static constexpr bool SUM = (MODE & FM_SUM) != 0;
     static constexpr bool MM = (MODE & FM_MM) != 0;
@@ -459,6 +458,57 @@ struct FastWarp {
     __device__ __forceinline__ void rows(const bool (&act)[U], const uint64_t (&kw)[U], const VT (&v)[U], unsigned lane) {
         const bool no[U] = {};
         rows<U>(act, kw, v, no, no, lane);
+    }
+
+    // U rows per lane of a table that holds every group (no NULLs): the common row finds its key in its home bucket, and
+    // everything else is worked out only in steps that hold such a row.  (In a spilling table, where most steps hold a
+    // miss, that order costs a quarter more than rows(): 2.18 against 1.66 ms for 2^28 rows.)
+    template <int U>
+    __device__ __forceinline__ void rows_fit(const bool (&act)[U], const uint64_t (&kw)[U], const VT (&v)[U]) {
+        long long q[U];
+        bool look[U], hit[U], any_miss = false;
+        uint64_t m[U];
+        uint32_t b[U], slot[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            look[u] = true;
+            q[u] = 0;
+            if constexpr (SUM) q[u] = addq<VT>(v[u], fq, look[u]);
+            look[u] = look[u] & act[u];
+            if constexpr (!K32) look[u] = look[u] & (kw[u] != kEmpty);
+            m[u] = fhash(kw[u]);
+            b[u] = fbucket(m[u], bshift, t.NB);
+        }
+        {
+            uint64_t k0[U], k1[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) lds128(t.keys + b[u] * 16u, k0[u], k1[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const bool h0 = k0[u] == kw[u];
+                hit[u] = look[u] & (h0 | (k1[u] == kw[u]));
+                slot[u] = h0 ? b[u] : t.NB + b[u];
+                any_miss |= act[u] & !hit[u];
+            }
+        }
+        if (__any_sync(0xffffffffu, any_miss)) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (look[u] && !hit[u]) {
+                    bool e = false;
+                    int s2 = fprobe(t, falt(m[u], t.NB), kw[u], e);  // a key whose home bucket is full
+                    if (s2 < 0) s2 = fclaim(t, b[u], kw[u], probe_b);
+                    hit[u] = s2 >= 0;
+                    slot[u] = static_cast<uint32_t>(s2);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (act[u] && !hit[u]) global_row(kw[u], v[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (hit[u]) update(slot[u], q[u], v[u]);
     }
 
     // U rows per lane: (act[u], kw[u], v[u]) (FM_NULL: vn[u] its value is NULL, esc[u] kw[u] is a real key
@@ -914,6 +964,7 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
                 vn = ring_bit(sl.vnull, g);
             } else if constexpr (COMP) kw = composite_word(static_cast<int32_t>(rk0[g]), static_cast<int32_t>(rk1[g]));
             else if constexpr (KZ) kw = key_word(kz_ring<KT>(ring + sl.key0, kzb, g, a.kz_off));
+            else if constexpr (KMOD) kw = key_word(kmod_key<KT>(a, rk0[g]));  // of passing rows only
             else kw = key_word(rk0[g]);
             if constexpr (VALS) v = rv[g];
             else v = VT{};
@@ -1012,20 +1063,6 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
             // The next tile of this CTA is staged too: rows left over may wait for it.
             const bool keep_going = carry && !full && q + 1 < my_tiles && tile + gridDim.x < a.full_tiles;
             const int g0 = s * kFastT + warp * kFastR;  // ring index of the warp's first row in this stage
-            if constexpr (KMOD) {
-                if (!full) {
-                    // Fused key % m: the warp replaces its own rows' keys in the stage by their remainders (no other
-                    // warp reads them), then fences its writes against the producer's next copy into the stage.
-                    KT* wk = const_cast<KT*>(rk0);
-#pragma unroll
-                    for (int j = 0; j < kFastSeg; ++j) {
-                        const int g = g0 + 32 * j + lane;
-                        wk[g] = static_cast<KT>(mod_signed(static_cast<int64_t>(wk[g]), a.km_d, a.km_m, a.km_s1, a.km_s2));
-                    }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    __syncwarp();
-                }
-            }
             int total = lc;
             if (!full) {
                 if (NUL && !listed) {
@@ -1411,6 +1448,12 @@ int32_t launch_fast_i32_nul(const AggArgs& a, ValKind vk, size_t smem, cudaStrea
 int32_t launch_fast_i64_nul(const AggArgs& a, ValKind vk, size_t smem, cudaStream_t st);
 int32_t launch_fast_f32_nul(const AggArgs& a, ValKind vk, size_t smem, cudaStream_t st);
 int32_t launch_fast_f64_nul(const AggArgs& a, ValKind vk, size_t smem, cudaStream_t st);
+// The pass of tables that hold every group (groupby_few.cuh): `grid` CTAs.
+int32_t launch_few_i32(const AggArgs& a, ValKind vk, size_t smem, int64_t grid, cudaStream_t st);
+int32_t launch_few_i64(const AggArgs& a, ValKind vk, size_t smem, int64_t grid, cudaStream_t st);
+int32_t launch_few_f32(const AggArgs& a, ValKind vk, size_t smem, int64_t grid, cudaStream_t st);
+int32_t launch_few_f64(const AggArgs& a, ValKind vk, size_t smem, int64_t grid, cudaStream_t st);
+int32_t launch_few_comp(const AggArgs& a, ValKind vk, size_t smem, int64_t grid, cudaStream_t st);
 int32_t launch_fast_comp(const AggArgs& a, ValKind vk, int32_t ptype, size_t smem, cudaStream_t st);
 
 }  // namespace qdb

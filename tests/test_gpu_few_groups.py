@@ -1,0 +1,84 @@
+"""The aggregation pass of tables that hold every group (no ring, no spill), against the oracle: every key and value type
+at the edges of its steps (2 or 4 rows a thread, 768 threads, one CTA per SM), predicates of every type, keys that never
+enter a shared table, values outside the fixed-point window, and tables up to the most groups the pass takes."""
+import numpy as np
+import pytest
+
+import oracle
+from gpu_compare import compare
+from qikkdb_b200 import datagen as dg
+from qikkdb_b200.groupby import (GPU_HASH_TABLE_FULL, FilterConditions, GroupByTable, QueryEngineError, make_pred,
+                                 process_mod)
+from test_gpu_masked import _keys, _vals
+from test_gpu_parity import ALL, _dev, run_both
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [2048, 2049, 3071, 3073, 1536 * 148 + 1, 3072 * 148 - 1, 3072 * 148 * 2 + 5])
+@pytest.mark.parametrize("kdt", [np.int32, np.int64, np.float32, np.float64])
+@pytest.mark.parametrize("vdt", [np.int32, np.int64, np.float32, np.float64])
+def test_few_groups(cuda, n, kdt, vdt):
+    rng = np.random.default_rng([n, np.dtype(kdt).num, np.dtype(vdt).num])
+    groups = (3, 90, 1500)[n % 3]
+    k, v = _keys(rng, n, groups, kdt), _vals(rng, n, vdt)
+    vf, kf = vdt in (np.float32, np.float64), kdt in (np.float32, np.float64)
+    kw = dict(val_is_float=vf, key_is_float=kf)
+    cap = groups + 3
+    run_both(k, v, ALL, cap, **kw)
+    run_both(k, v, ["sum"], cap, blocks=2 if n > 6000 else 1, **kw)
+    run_both(k, v, ["max"], cap, **kw)
+    run_both(k, v, ["count"], cap, **kw)
+    pcol = rng.integers(0, 100, n).astype((np.int32, np.int64, np.float32, np.float64)[n % 4])
+    for op, c in ((FilterConditions.less, 60), (FilterConditions.notEqual, 7), (FilterConditions.greater, 99)):
+        run_both(k, v, ["sum", "min", "count"], cap, pred=(pcol, op, c, np.int32, None), **kw)
+
+
+@pytest.mark.parametrize("n", [2048, 4099, 1_000_003])
+@pytest.mark.parametrize("side", [2, 40])
+def test_few_groups_composite(cuda, n, side):
+    rng = np.random.default_rng(n + side)
+    a, b = (rng.integers(-side, side, n).astype(np.int32) for _ in range(2))
+    a[rng.random(n) < 0.01] = np.iinfo(np.int32).min  # with b == 0: the empty slot's word
+    run_both([a, b], rng.integers(-(1 << 40), 1 << 40, n), ALL, 4 * side * side + 2 * side)
+    run_both([a, b], np.exp(rng.standard_normal(n)), ["sum", "avg"], 4 * side * side + 2 * side, val_is_float=True)
+
+
+@pytest.mark.parametrize("groups", [2700, 3500, 5600, 5850])
+def test_few_groups_up_to_the_largest_table(cuda, groups):
+    """Around the group counts where the table stops fitting and the call takes the spilling pass."""
+    n = 800_001
+    k = dg.uniform_i32(5, groups, n, 0, groups - 1) * 7919
+    v = dg.uniform_i32(6, groups, n, -1000, 1000)
+    run_both(k, v, ["sum", "count"], groups)
+    run_both(k, v, ALL, groups)
+
+
+@pytest.mark.parametrize("kdt", [np.int32, np.int64])
+@pytest.mark.parametrize("m", [1, 7, -30, 1000, 2600, 4000])
+def test_few_groups_modulo(cuda, kdt, m):
+    """GROUP BY key % m: few remainders take this pass, more the spilling one, which takes the remainder of the passing
+    rows' keys as it reads them."""
+    n = 700_003
+    rng = np.random.default_rng(abs(m))
+    info = np.iinfo(kdt)
+    k = rng.integers(info.min, info.max, n, dtype=kdt)
+    v = rng.integers(-1000, 1000, n).astype(np.int64)
+    p = rng.random(n).astype(np.float32)
+    t = GroupByTable(["sum", "count"], kdt, np.int64, 2 * abs(m))
+    process_mod(t, _dev(k), m, _dev(v), make_pred(_dev(p), FilterConditions.less, 0.3, np.float32))
+    rem = np.fmod(k.astype(np.int64), m)
+    r = oracle.groupby(rem, v, pred=(p, FilterConditions.less, 0.3, np.float32, None))
+    compare(t.results_numpy(), r, ["sum", "count"], False)
+
+
+def test_few_groups_table_full(cuda):
+    k = dg.uniform_i32(7, 0, 100_000, 0, 999)
+    t = GroupByTable(["sum"], np.int32, np.int32, 400)
+    with pytest.raises(QueryEngineError) as e:
+        t.process([_dev(k)], _dev(k), len(k))
+    assert e.value.code == GPU_HASH_TABLE_FULL
+    r = oracle.groupby(k % 400, k)
+    t.reset()
+    t.process([_dev(k % 400)], _dev(k), len(k))
+    assert t.results_numpy()["n_groups"] == r["count"] == 400
