@@ -1,9 +1,10 @@
 // Result extraction of a GROUP BY table: the GetResults pass (qikkDB/QueryEngine/GPUCore/GPUGroupBy.cuh:478-587,
 // GPUGroupByMultiKey.cuh:742-912).  The reference builds an occupancy mask, compacts keys with a CUB scan,
 // folds 256 value replicas per slot, divides for AVG and compacts again.  Here the table has no replicas, so
-// the pass is: count occupied slots per 4096-slot chunk, scan the chunk counts, and emit every output column
+// the pass is: count occupied slots per chunk of slots, scan the chunk counts, and emit every output column
 // (keys, key null bits, each requested aggregate with its null bits) in one kernel that finalises AVG and the
 // NULL conventions on the fly.  Output order is slot order, like the reference's.
+#include <algorithm>
 #include <limits>
 #include <vector>
 
@@ -12,9 +13,6 @@
 namespace qdb {
 
 constexpr int kResThreads = 256;
-constexpr int kResPerThread = 16;
-constexpr int kResChunk = kResThreads * kResPerThread;
-
 // Block-wide exclusive scan of one int per thread (kResThreads threads).
 __device__ __forceinline__ int block_excl_scan(int x, int* total) {
     __shared__ int warp_sums[kResThreads / 32];
@@ -44,17 +42,26 @@ __device__ __forceinline__ int block_excl_scan(int x, int* total) {
     return excl;
 }
 
-// A chunk's slots are walked warp by warp: warp w of the block takes the kResWarpSlots consecutive slots from
-// chunk start + w kResWarpSlots, 32 at a time (one slot per lane), so every load of the key words is coalesced.
-constexpr int kResWarpSlots = kResChunk / (kResThreads / 32);
+// A chunk's slots are walked warp by warp: warp w of the block takes the ws consecutive slots from chunk start + w ws,
+// 32 at a time (one slot per lane), so every load of the key words is coalesced.  ws is a multiple of 32: 512 for large
+// tables, less for tables that would leave SMs without a chunk (a warp's steps are a chain of dependent loads: 1000
+// groups in one chunk of 4096 slots took 28 us to emit, now spread over eight blocks).
+constexpr int kResWarps = kResThreads / 32;
+constexpr int kResMaxWarpSlots = 512;
+
+static int res_warp_slots(uint64_t total) {
+    const uint64_t blocks = 2 * static_cast<uint64_t>(device_info().sm_count);
+    const uint64_t per = (total + blocks * kResWarps - 1) / (blocks * kResWarps);
+    return static_cast<int>(std::min<uint64_t>(kResMaxWarpSlots, std::max<uint64_t>(32, (per + 31) / 32 * 32)));
+}
 
 // A table of one chunk needs no scan: its offset is 0 and its count the total.
-__global__ void res_count_kernel(SlotSpace sp, int* chunk_counts, long long* total_out) {
+__global__ void res_count_kernel(SlotSpace sp, int ws, int* chunk_counts, long long* total_out) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint64_t wbase = static_cast<uint64_t>(blockIdx.x) * kResChunk + static_cast<uint64_t>(warp) * kResWarpSlots;
+    const uint64_t wbase = (static_cast<uint64_t>(blockIdx.x) * kResWarps + warp) * static_cast<uint64_t>(ws);
     int c = 0;
 #pragma unroll 4
-    for (int i = 0; i < kResWarpSlots; i += 32) c += present(sp, wbase + i + lane) ? 1 : 0;
+    for (int i = 0; i < ws; i += 32) c += present(sp, wbase + i + lane) ? 1 : 0;
     __shared__ int tot;
     block_excl_scan(c, &tot);
     if (threadIdx.x == 0) {
@@ -102,6 +109,7 @@ struct EmitArgs {
     int32_t n_out = 0;
     OutAgg out[5];
     const int* chunk_offsets = nullptr;
+    int ws = 0;  // slots per warp of a chunk
 };
 
 __device__ __forceinline__ void set_bit(unsigned long long* m, int64_t pos) {
@@ -247,17 +255,18 @@ __device__ void res_emit_one(const EmitArgs& a, uint64_t v, int64_t pos) {
 }
 
 __global__ void res_emit_kernel(EmitArgs a) {
+    const int ws = a.ws;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint64_t wbase = static_cast<uint64_t>(blockIdx.x) * kResChunk + static_cast<uint64_t>(warp) * kResWarpSlots;
+    const uint64_t wbase = (static_cast<uint64_t>(blockIdx.x) * kResWarps + warp) * static_cast<uint64_t>(ws);
     // the warp's present slots, then its offset in the chunk (an exclusive scan of the warp counts)
     int c = 0;
 #pragma unroll 4
-    for (int i = 0; i < kResWarpSlots; i += 32) c += __popc(__ballot_sync(0xffffffffu, present(a.sp, wbase + i + lane)));
+    for (int i = 0; i < ws; i += 32) c += __popc(__ballot_sync(0xffffffffu, present(a.sp, wbase + i + lane)));
     __shared__ int tot;
     int64_t pos = a.chunk_offsets[blockIdx.x] + block_excl_scan(lane == 0 ? c : 0, &tot);
     pos = __shfl_sync(0xffffffffu, pos, 0);
     const unsigned lt = (1u << lane) - 1u;
-    for (int i = 0; i < kResWarpSlots; i += 32) {
+    for (int i = 0; i < ws; i += 32) {
         const uint64_t v = wbase + i + lane;
         const bool pr = present(a.sp, v);
         const unsigned bal = __ballot_sync(0xffffffffu, pr);
@@ -303,13 +312,15 @@ int32_t qdb_gb_results_multi(qdb_gb* gb, int32_t n_aggs, const int32_t* aggs, vo
     cudaStream_t s = as_stream(stream);
 
     const SlotSpace sp = slot_space(gb);
-    const int64_t nchunks = static_cast<int64_t>((sp.total + kResChunk - 1) / kResChunk);
+    const int ws = res_warp_slots(sp.total);
+    const uint64_t chunk = static_cast<uint64_t>(kResWarps) * ws;
+    const int64_t nchunks = static_cast<int64_t>((sp.total + chunk - 1) / chunk);
 
     long long* d_total = nullptr;  // the group count, then the chunk counts
     int32_t rc = dev_alloc(reinterpret_cast<void**>(&d_total), sizeof(long long) + (nchunks + 1) * sizeof(int), s);
     if (rc != QDB_OK) return rc;
     int* counts = reinterpret_cast<int*>(d_total + 1);
-    res_count_kernel<<<static_cast<unsigned>(nchunks), kResThreads, 0, s>>>(sp, counts, d_total);
+    res_count_kernel<<<static_cast<unsigned>(nchunks), kResThreads, 0, s>>>(sp, ws, counts, d_total);
     note_launch();
     if (nchunks > 1) {
         res_scan_kernel<<<1, kResThreads, 0, s>>>(counts, nchunks, d_total);
@@ -340,6 +351,7 @@ int32_t qdb_gb_results_multi(qdb_gb* gb, int32_t n_aggs, const int32_t* aggs, vo
     ea.composite = gb->n_key_cols == 2;
     ea.vk = vk;
     ea.chunk_offsets = counts;
+    ea.ws = ws;
     ea.n_out = n_aggs;
     for (int c = 0; c < nk && rc == QDB_OK; ++c) {
         rc = alloc(&out_keys[c], static_cast<size_t>(total) * ksize);
