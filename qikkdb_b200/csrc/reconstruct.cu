@@ -5,8 +5,13 @@
 // The reference runs a CUB InclusiveSum of the int8 mask into an int32 array (4 B/row written and read
 // back), reads the count back, allocates, and scatters with kernel_reconstruct_col.  Here a pass counts
 // the selected rows of every 4096-row tile (1 B/row read), one block scans the tile counts, and the
-// scatter pass recomputes each thread's offset inside its tile from the mask (a block scan in registers
+// scatter pass recomputes each warp's offset inside its tile from the mask (a block scan in registers
 // and shared memory), so no per-row prefix array touches HBM.  No pass waits on another CTA.
+//
+// The scatter is bound by memory.  A warp takes 512 consecutive rows, 32 at a time: a lane reads 16 mask bytes in one
+// load, and the two lanes that hold a step's bits hand them to all, so the column is read and written in whole lines.
+// (With 16 consecutive rows per thread every load and store instruction touched 32 lines: 33M rows, 30 % kept, 95 us
+// for an 8-byte and 67 us for a 4-byte column, now 67 and 50 us.)
 #include <mutex>
 #include <string>
 #include <vector>
@@ -73,17 +78,24 @@ __global__ void rc_count_kernel(const int8_t* __restrict__ mask, int64_t n, int 
     if (threadIdx.x == 0) tile_counts[blockIdx.x] = tot;
 }
 
-// Exclusive scan of tile counts in one block; tile_counts[ntiles] receives the total.
-__global__ void rc_scan_kernel(long long* tile_counts, int64_t ntiles) {
-    __shared__ long long carry;
-    __shared__ long long wsum[kRcThreads / 32];
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
+// Exclusive scan of tile counts in one block, kRcScanPer consecutive counts per thread and step; tile_counts[ntiles]
+// receives the total.
+constexpr int kRcScanThreads = 1024;
+constexpr int kRcScanPer = 8;
+__global__ void __launch_bounds__(kRcScanThreads) rc_scan_kernel(long long* tile_counts, int64_t ntiles) {
+    __shared__ long long wsum[kRcScanThreads / 32];
+    __shared__ long long s_all;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int64_t base = 0; base < ntiles; base += kRcThreads) {
-        const int64_t i = base + threadIdx.x;
-        const long long x = (i < ntiles) ? tile_counts[i] : 0;
-        long long inc = x;
+    long long carry = 0;
+    for (int64_t base = 0; base < ntiles; base += kRcScanThreads * kRcScanPer) {
+        const int64_t i0 = base + static_cast<int64_t>(threadIdx.x) * kRcScanPer;
+        long long x[kRcScanPer], sum = 0;
+#pragma unroll
+        for (int k = 0; k < kRcScanPer; ++k) {
+            x[k] = i0 + k < ntiles ? tile_counts[i0 + k] : 0;
+            sum += x[k];
+        }
+        long long inc = sum;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const long long y = __shfl_up_sync(0xffffffffu, inc, o);
@@ -91,14 +103,25 @@ __global__ void rc_scan_kernel(long long* tile_counts, int64_t ntiles) {
         }
         if (lane == 31) wsum[wid] = inc;
         __syncthreads();
-        long long before = 0, all = 0;
-        for (int w = 0; w < kRcThreads / 32; ++w) {
-            if (w < wid) before += wsum[w];
-            all += wsum[w];
+        if (wid == 0) {
+            const long long w = wsum[lane];
+            long long wi = w;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long y = __shfl_up_sync(0xffffffffu, wi, o);
+                if (lane >= o) wi += y;
+            }
+            wsum[lane] = wi - w;
+            if (lane == 31) s_all = wi;
         }
-        if (i < ntiles) tile_counts[i] = carry + before + inc - x;
         __syncthreads();
-        if (threadIdx.x == 0) carry += all;
+        long long run = carry + wsum[wid] + inc - sum;
+#pragma unroll
+        for (int k = 0; k < kRcScanPer; ++k) {
+            if (i0 + k < ntiles) tile_counts[i0 + k] = run;
+            run += x[k];
+        }
+        carry += s_all;
         __syncthreads();
     }
     if (threadIdx.x == 0) tile_counts[ntiles] = carry;
@@ -111,13 +134,33 @@ __global__ void rc_scatter_kernel(const T* __restrict__ in, const int8_t* __rest
     const int64_t base = static_cast<int64_t>(blockIdx.x) * kRcTile + threadIdx.x * kRcPerThread;
     const uint32_t bits = (base < n) ? mask_bits(mask, base, n, vec) : 0u;
     __shared__ int tot;
-    long long pos = tile_offsets[blockIdx.x] + rc_block_excl_scan(__popc(bits), &tot);
-    for (int e = 0; e < kRcPerThread; ++e) {
-        if (!((bits >> e) & 1u)) continue;
-        const int64_t r = base + e;
-        out[pos] = in[r];
-        if (null_out && null_bit(null_in, r)) atomicOr(null_out + (pos >> 6), 1ull << (pos & 63));
-        ++pos;
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    // the warp's first output position: lane 0's offset in the block
+    const int off = rc_block_excl_scan(__popc(bits), &tot);
+    long long pos = tile_offsets[blockIdx.x] + __shfl_sync(0xffffffffu, off, 0);
+    const int64_t row0 = base - static_cast<int64_t>(lane) * kRcPerThread + lane;  // this lane's row of step 0
+    constexpr int kHalf = kRcPerThread / 2;  // steps whose loads are in flight together
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t sel[kHalf];
+        T v[kHalf];
+#pragma unroll
+        for (int j = 0; j < kHalf; ++j) {
+            const int src = 2 * (h * kHalf + j);
+            sel[j] = __shfl_sync(0xffffffffu, bits, src) | (__shfl_sync(0xffffffffu, bits, src + 1) << 16);
+            if ((sel[j] >> lane) & 1u) v[j] = in[row0 + 32 * (h * kHalf + j)];
+        }
+#pragma unroll
+        for (int j = 0; j < kHalf; ++j) {
+            if ((sel[j] >> lane) & 1u) {
+                const long long p = pos + __popc(sel[j] & lt);
+                out[p] = v[j];
+                if (null_out && null_bit(null_in, row0 + 32 * (h * kHalf + j)))
+                    atomicOr(null_out + (p >> 6), 1ull << (p & 63));
+            }
+            pos += __popc(sel[j]);
+        }
     }
 }
 
@@ -127,9 +170,17 @@ __global__ void rc_indexes_kernel(const int8_t* __restrict__ mask, int64_t n, in
     const int64_t base = static_cast<int64_t>(blockIdx.x) * kRcTile + threadIdx.x * kRcPerThread;
     const uint32_t bits = (base < n) ? mask_bits(mask, base, n, vec) : 0u;
     __shared__ int tot;
-    long long pos = tile_offsets[blockIdx.x] + rc_block_excl_scan(__popc(bits), &tot);
-    for (int e = 0; e < kRcPerThread; ++e)
-        if ((bits >> e) & 1u) out[pos++] = static_cast<int32_t>(base + e);
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    const int off = rc_block_excl_scan(__popc(bits), &tot);
+    long long pos = tile_offsets[blockIdx.x] + __shfl_sync(0xffffffffu, off, 0);
+    const int64_t row0 = base - static_cast<int64_t>(lane) * kRcPerThread + lane;
+#pragma unroll
+    for (int j = 0; j < kRcPerThread; ++j) {
+        const uint32_t sel = __shfl_sync(0xffffffffu, bits, 2 * j) | (__shfl_sync(0xffffffffu, bits, 2 * j + 1) << 16);
+        if ((sel >> lane) & 1u) out[pos + __popc(sel & lt)] = static_cast<int32_t>(row0 + 32 * j);
+        pos += __popc(sel);
+    }
 }
 
 // Inclusive prefix sum of the mask (PrefixSum<int32_t,int8_t>).  Like CUB's InclusiveSum over int8 input
@@ -187,7 +238,7 @@ static int32_t count_and_scan(const int8_t* mask, int64_t n, bool sum_values, lo
     if (sum_values) rc_sum_kernel<<<static_cast<unsigned>(ntiles), kRcThreads, 0, s>>>(mask, n, *offsets);
     else rc_count_kernel<<<static_cast<unsigned>(ntiles), kRcThreads, 0, s>>>(mask, n, vec, *offsets);
     note_launch();
-    rc_scan_kernel<<<1, kRcThreads, 0, s>>>(*offsets, ntiles);
+    rc_scan_kernel<<<1, kRcScanThreads, 0, s>>>(*offsets, ntiles);
     note_launch();
     if (total) {
         const cudaError_t e = read_back(total, *offsets + ntiles, sizeof(long long), s);
@@ -404,7 +455,7 @@ extern "C" int32_t qdb_reconstruct_keep_noalloc(int32_t elem_bytes, const void* 
     // Every entry the scan reads is written by the count pass first, so the scratch needs no clearing.
     rc_count_kernel<<<static_cast<unsigned>(ntiles), kRcThreads, 0, s>>>(mask, n, vec, offs);
     note_launch();
-    rc_scan_kernel<<<1, kRcThreads, 0, s>>>(offs, ntiles);
+    rc_scan_kernel<<<1, kRcScanThreads, 0, s>>>(offs, ntiles);
     note_launch();
     long long total = 0;
     cudaError_t e = cudaMemcpyAsync(&total, offs + ntiles, sizeof(long long), cudaMemcpyDeviceToHost, s);
