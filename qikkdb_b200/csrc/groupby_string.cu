@@ -114,8 +114,23 @@ __device__ int64_t gbs_find(const GbsDict& t, const uint64_t* __restrict__ W, in
     }
     const bool shortk = n <= 8 * kGbsInline;
     uint64_t w[kGbsInline];
+    if (shortk) {
+        // The aligned words that hold the key, each loaded once, then shifted together.
+        const int64_t k = b >> 3, last = n > 0 ? (b + n - 1) >> 3 : k - 1;
+        const int sh = static_cast<int>(b & 7) * 8;
+        uint64_t x[kGbsInline + 1];
 #pragma unroll
-    for (int j = 0; j < kGbsInline; ++j) w[j] = 8 * j < n ? gbs_word(W, b + 8 * j, n - 8 * j) : 0ull;
+        for (int j = 0; j <= kGbsInline; ++j) x[j] = k + j <= last ? __ldg(W + k + j) : 0ull;
+#pragma unroll
+        for (int j = 0; j < kGbsInline; ++j) {
+            w[j] = sh ? (x[j] >> sh) | (x[j + 1] << (64 - sh)) : x[j];
+            const int64_t take = n - 8 * j;  // bytes of the key in this word
+            if (take < 8) w[j] = take > 0 ? w[j] & ((1ull << (8 * take)) - 1ull) : 0ull;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < kGbsInline; ++j) w[j] = gbs_word(W, b + 8 * j, n - 8 * j);
+    }
     uint64_t h = 0x243F6A8885A308D3ull ^ (static_cast<uint64_t>(n) * 0xBF58476D1CE4E5B9ull);
 #pragma unroll
     for (int j = 0; j < kGbsInline; ++j)
@@ -126,6 +141,16 @@ __device__ int64_t gbs_find(const GbsDict& t, const uint64_t* __restrict__ W, in
     const int64_t words = (n + 7) >> 3;
     const uint64_t mask = t.cap - 1;
     uint64_t pos = __umul64hi(h, t.cap);
+    if (shortk) {
+        // Most rows find their key's record in its home slot: comparing the key itself there spares them the header, a
+        // dependent load of the chain that this pass is bound by.  Anything else takes the full probe below.
+        // One 32-byte load, so meta and words are of one time; meta 0 (unpublished) or poison never matches a length.
+        uint64_t m, r0, r1, r2;
+        asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                     : "=l"(m), "=l"(r0), "=l"(r1), "=l"(r2) : "l"(t.rec + pos) : "memory");
+        if (m != kMetaPoison && gbs_meta_len(m) == n && ((r0 == w[0]) & (r1 == w[1]) & (r2 == w[2])))
+            return static_cast<int64_t>(pos);
+    }
     for (uint64_t probe = 0; probe < t.cap; ++probe, pos = (pos + 1) & mask) {
         uint64_t cur = t.header[pos];  // a stale 0 only sends the row to the CAS, which reads the live value
         GbsRec* r = t.rec + pos;
