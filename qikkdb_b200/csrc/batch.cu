@@ -14,6 +14,7 @@ namespace qdb {
 
 __global__ void gb_batch_init_kernel(const BatchArgs ba);
 __global__ void gb_batch_agg_kernel(const BatchArgs ba);
+__global__ void gb_batch_count_kernel(const BatchArgs ba);
 __global__ void gb_batch_results_kernel(const BatchArgs ba);
 
 // A plan family the autotuner chooses between, independent of one query's sizes.
@@ -88,6 +89,7 @@ struct qdb_gb_batch {
     uint64_t* d_res = nullptr;
     unsigned long long* d_counters = nullptr;
     int64_t* d_res_count = nullptr;
+    int32_t* d_res_chunks = nullptr;    // behind d_res_count
     int32_t* d_status = nullptr;
     long long* d_item_ns = nullptr;
     // pinned host staging
@@ -129,6 +131,7 @@ static BatchArgs batch_args(const qdb_gb_batch* b) {
     a.groups = b->d_groups;
     a.res = b->d_res;
     a.res_count = b->d_res_count;
+    a.res_chunks = b->d_res_chunks;
     a.status = b->d_status;
     a.item_ns = b->d_item_ns;
     a.dyn_bytes = static_cast<int64_t>(b->dyn_bytes);
@@ -356,11 +359,17 @@ static int32_t wait_staging(qdb_gb_batch* b) {
     return QDB_OK;
 }
 
+static void launch_results(const qdb_gb_batch* b, BatchArgs a, cudaStream_t s) {
+    const dim3 grid(static_cast<unsigned>(b->max_inst), kBResBlocks);
+    gb_batch_count_kernel<<<grid, kBResThreads, 0, s>>>(a);
+    gb_batch_results_kernel<<<grid, kBResThreads, 0, s>>>(a);
+}
+
 static int32_t launch_all(qdb_gb_batch* b, cudaStream_t s) {
     const BatchArgs a = batch_args(b);
     gb_batch_init_kernel<<<static_cast<unsigned>(b->max_inst), 1024, 0, s>>>(a);
     gb_batch_agg_kernel<<<static_cast<unsigned>(b->grid), kBThreads, b->dyn_bytes, s>>>(a);
-    gb_batch_results_kernel<<<static_cast<unsigned>(b->max_inst), kBResThreads, 0, s>>>(a);
+    launch_results(b, a, s);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "batch kernels launch");
     return QDB_OK;
@@ -441,7 +450,7 @@ static int32_t run_once(qdb_gb_batch* b, bool use_graph, cudaStream_t s) {
             const BatchArgs a = batch_args(b);
             gb_batch_init_kernel<<<static_cast<unsigned>(b->max_inst), 1024, 0, s>>>(a);
             gb_batch_agg_kernel<<<static_cast<unsigned>(b->grid), kBThreads, b->dyn_bytes, s>>>(a);
-            gb_batch_results_kernel<<<static_cast<unsigned>(b->max_inst), kBResThreads, 0, s>>>(a);
+            launch_results(b, a, s);
             cudaGraph_t g = nullptr;
             cudaError_t e = cudaStreamEndCapture(s, &g);
             if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture(batch)");
@@ -457,7 +466,7 @@ static int32_t run_once(qdb_gb_batch* b, bool use_graph, cudaStream_t s) {
         int32_t rc = launch_all(b, s);
         if (rc != QDB_OK) return rc;
     }
-    note_launch(3);
+    note_launch(4);
     b->needs_init = false;
     return QDB_OK;
 }
@@ -527,7 +536,11 @@ int32_t qdb_gb_batch_create(qdb_gb_batch** out, int32_t max_instances, int64_t t
     if (table_bytes > 0) try_cuda(cudaMalloc(&b->d_tables, table_bytes), "cudaMalloc(batch tables)");
     if (result_bytes > 0) try_cuda(cudaMalloc(&b->d_res, result_bytes), "cudaMalloc(batch results)");
     try_cuda(cudaMalloc(&b->d_counters, 2 * max_instances * sizeof(unsigned long long)), "cudaMalloc(batch counters)");
-    try_cuda(cudaMalloc(&b->d_res_count, max_instances * sizeof(int64_t)), "cudaMalloc(batch counts)");
+    // the group counts, then the chunk counts: a chunk holds kBResChunk slots of at least 8 bytes, and every query may
+    // add a partial one
+    const int64_t chunks = max_instances + table_bytes / (kBResChunk * 8) + 1;
+    try_cuda(cudaMalloc(&b->d_res_count, max_instances * sizeof(int64_t) + chunks * sizeof(int32_t)), "cudaMalloc(batch counts)");
+    b->d_res_chunks = reinterpret_cast<int32_t*>(b->d_res_count + max_instances);
     try_cuda(cudaMalloc(&b->d_status, max_instances * sizeof(int32_t)), "cudaMalloc(batch status)");
     try_cuda(cudaMallocHost(&b->h_hdr, sizeof(BHeader)), "cudaMallocHost(batch header)");
     try_cuda(cudaMallocHost(&b->h_inst, max_instances * sizeof(BInst)), "cudaMallocHost(batch descriptors)");
@@ -581,7 +594,7 @@ int32_t qdb_gb_batch_set(qdb_gb_batch* b, const qdb_gb_query* queries, int32_t n
     if (!b) return fail(QDB_ERR_INVALID, "qdb_gb_batch_set: null batch");
     if (n < 0 || n > b->max_inst || (n > 0 && !queries)) return fail(QDB_ERR_INVALID, "qdb_gb_batch_set: bad query count");
     std::vector<qdb_gb_query> qs(queries, queries + n);
-    int64_t table_off = 0, res_off = 0, total_rows = 0;
+    int64_t table_off = 0, res_off = 0, total_rows = 0, chunk0 = 0;
     std::vector<int64_t> toff(n), roff(n);
     for (int i = 0; i < n; ++i) {
         int32_t rc = check_query(qs[i]);
@@ -624,6 +637,8 @@ int32_t qdb_gb_batch_set(qdb_gb_batch* b, const qdb_gb_query* queries, int32_t n
         I.capacity = q.max_groups;
         I.res_off = roff[i] / 8;
         I.res_cap = q.max_groups + 2;
+        I.res_chunk0 = chunk0;
+        chunk0 += static_cast<int64_t>((cap + 2 + kBResChunk - 1) / kBResChunk);
         I.L = make_layout(q.agg_mask, vk);
         I.kt = q.key_type == QDB_INT64 ? 8 : 4;
         I.vk = vk;

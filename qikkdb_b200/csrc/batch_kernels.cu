@@ -829,8 +829,37 @@ __device__ uint64_t b_emit(const BInst& I, const uint64_t* slot, int agg) {
     }
 }
 
+// A chunk's slots are walked warp by warp (warp w: kBResWarp consecutive slots, one per lane per step), so the key-word
+// loads are coalesced.
+constexpr int kBResWarp = kBResChunk / (kBResThreads / 32);
+
+// Groups present in every chunk of every query (grid: queries x kBResBlocks).
+__global__ void __launch_bounds__(kBResThreads) gb_batch_count_kernel(const BatchArgs ba) {
+    const int i = blockIdx.x;
+    if (i >= ba.hdr->n_inst) return;
+    const BInst& I = ba.inst[i];
+    const uint64_t total = I.main.mask + 3;
+    const int W = I.L.W;
+    const uint64_t* slots = I.main.slots;
+    const uint64_t nch = (total + kBResChunk - 1) / kBResChunk;
+    __shared__ int tot_s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (uint64_t ch = blockIdx.y; ch < nch; ch += kBResBlocks) {
+        const uint64_t wb = ch * kBResChunk + static_cast<uint64_t>(warp) * kBResWarp;
+        int c = 0;
+#pragma unroll
+        for (int k = 0; k < kBResWarp; k += 32) {
+            const uint64_t v = wb + k + lane;
+            c += __popc(__ballot_sync(0xffffffffu, v < total && slots[v * W] != kEmpty));
+        }
+        b_block_scan(lane == 0 ? c : 0, &tot_s);
+        if (threadIdx.x == 0) ba.res_chunks[I.res_chunk0 + ch] = tot_s;
+        __syncthreads();
+    }
+}
+
 __global__ void __launch_bounds__(kBResThreads) gb_batch_results_kernel(const BatchArgs ba) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
         for (int q = 0; q < kBQueues; ++q) ba.hdr->heads[q] = 0;
         ba.hdr->init_needed = 0;
     }
@@ -842,24 +871,31 @@ __global__ void __launch_bounds__(kBResThreads) gb_batch_results_kernel(const Ba
     const Layout L = I.L;
     uint64_t* res = ba.res + I.res_off;
     const int64_t cap = I.res_cap;
+    const int32_t* counts = ba.res_chunks + I.res_chunk0;
+    const uint64_t nch = (total + kBResChunk - 1) / kBResChunk;
     __shared__ int tot_s;
-    int64_t done = 0;
-    // A chunk's slots are walked warp by warp (warp w: kWS consecutive slots, one per lane per step), so the key-word
-    // loads are coalesced; a row's position is the chunk's base, its warp's offset and its rank in the ballot.
-    constexpr int kWS = kBResChunk / (kBResThreads / 32);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    for (uint64_t c0 = 0; c0 < total; c0 += kBResChunk) {
-        const uint64_t wb = c0 + static_cast<uint64_t>(warp) * kWS;
+    // A row's position is the counts of the chunks before, its warp's offset and its rank in the ballot.
+    int64_t before = 0;
+    uint64_t summed = 0;
+    for (uint64_t ch = blockIdx.y; ch < nch; ch += kBResBlocks) {
+        int part = 0;
+        for (uint64_t k = summed + threadIdx.x; k < ch; k += kBResThreads) part += counts[k];
+        b_block_scan(part, &tot_s);
+        before += tot_s;
+        summed = ch;
+        __syncthreads();
+        const uint64_t wb = ch * kBResChunk + static_cast<uint64_t>(warp) * kBResWarp;
         int c = 0;
-#pragma unroll 4
-        for (int k = 0; k < kWS; k += 32) {
+#pragma unroll
+        for (int k = 0; k < kBResWarp; k += 32) {
             const uint64_t v = wb + k + lane;
             c += __popc(__ballot_sync(0xffffffffu, v < total && I.main.slots[v * W] != kEmpty));
         }
-        int64_t pos = done + b_block_scan(lane == 0 ? c : 0, &tot_s);
+        int64_t pos = before + b_block_scan(lane == 0 ? c : 0, &tot_s);
         pos = __shfl_sync(0xffffffffu, pos, 0);
-        for (int k = 0; k < kWS; k += 32) {
+        for (int k = 0; k < kBResWarp; k += 32) {
             const uint64_t v = wb + k + lane;
             const bool pr = v < total && I.main.slots[v * W] != kEmpty;
             const unsigned bal = __ballot_sync(0xffffffffu, pr);
@@ -892,17 +928,17 @@ __global__ void __launch_bounds__(kBResThreads) gb_batch_results_kernel(const Ba
             }
             pos += __popc(bal);
         }
-        done += tot_s;
         __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        int32_t st = static_cast<int32_t>(I.counters[1] & 0xffffffffull);
-        if (ba.hdr->error != QDB_OK) st = ba.hdr->error;
-        if (done > cap && st == QDB_OK) st = QDB_HASH_TABLE_FULL;
-        ba.res_count[i] = done < cap ? done : cap;
-        ba.status[i] = st;
-        I.counters[0] = 0;
-        I.counters[1] = 0;
+        if (ch == nch - 1 && threadIdx.x == 0) {  // the query's last chunk: its count and status
+            const int64_t done = before + counts[ch];
+            int32_t st = static_cast<int32_t>(I.counters[1] & 0xffffffffull);
+            if (ba.hdr->error != QDB_OK) st = ba.hdr->error;
+            if (done > cap && st == QDB_OK) st = QDB_HASH_TABLE_FULL;
+            ba.res_count[i] = done < cap ? done : cap;
+            ba.status[i] = st;
+            I.counters[0] = 0;
+            I.counters[1] = 0;
+        }
     }
 }
 
