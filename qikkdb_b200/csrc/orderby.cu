@@ -76,7 +76,7 @@ __device__ __forceinline__ uint32_t ob_peers(uint32_t* words, uint32_t d, bool i
 // ---------------------------------------------------------------------------------------------
 // One block, every column.  Warp w holds positions [256 w, 256 w + 256), step j the positions 32 j + lane, so rows are
 // ranked in their order.  A digit that is the same in all rows is skipped.  n <= 8192 rows of 64-bit keys take 64 KB of
-// keys and 16 KB of row numbers; the time is the serial chain of the passes (about 2 us each), which is still far below
+// keys and 32 KB of row numbers; the time is the serial chain of the passes (about 2 us each), which is still far below
 // the launches of the tiled form: 1000 rows of one int32 column take one launch of 8 us instead of 13 launches, 31 us.
 // ---------------------------------------------------------------------------------------------
 struct ObSmallCol {
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(kObSmallThreads) ob_small_kernel(const ObSmall
     extern __shared__ __align__(16) unsigned char ob_sm[];
     const int warps = blockDim.x >> 5;
     uint64_t* keys = reinterpret_cast<uint64_t*>(ob_sm);                            // [blockDim.x * 8]
-    uint16_t* perm = reinterpret_cast<uint16_t*>(keys + blockDim.x * kObSmallItems);  // [blockDim.x * 8]
+    int32_t* perm = reinterpret_cast<int32_t*>(keys + blockDim.x * kObSmallItems);    // [blockDim.x * 8]
     uint32_t* words = reinterpret_cast<uint32_t*>(perm + blockDim.x * kObSmallItems); // [warps][256] lane masks
     uint16_t* cnt = reinterpret_cast<uint16_t*>(words + warps * 256);                 // [warps][256]
     __shared__ uint32_t s_vary[2];
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kObSmallThreads) ob_small_kernel(const ObSmall
     for (int i = threadIdx.x; i < warps * 256; i += blockDim.x) words[i] = 0u;
     for (int j = 0; j < kObSmallItems; ++j) {
         const int i = i0 + 32 * j;
-        if (i < a.n) perm[i] = static_cast<uint16_t>(a.first ? i : a.idx[i]);
+        if (i < a.n) perm[i] = a.first ? i : a.idx[i];  // any row numbers of the columns, not only 0..n-1
     }
     for (int c = 0; c < a.n_cols; ++c) {
         const ObSmallCol& col = a.c[c];
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kObSmallThreads) ob_small_kernel(const ObSmall
             }
         };
         uint64_t key[kObSmallItems];
-        uint16_t id[kObSmallItems];
+        int32_t id[kObSmallItems];
         const uint64_t k0 = key_at(perm[0]);
         uint64_t vary = 0;
 #pragma unroll
@@ -578,7 +578,7 @@ static int32_t ob_column(const void* col, const uint64_t* nulls, int32_t desc, i
 static int32_t ob_small(const ObSmallArgs& a, cudaStream_t s) {
     const int per = 32 * kObSmallItems;
     const int threads = std::max(4, (a.n + per - 1) / per) * 32;  // at least four warps share the digit scans
-    const size_t smem = static_cast<size_t>(threads) * kObSmallItems * 10 + static_cast<size_t>(threads / 32) * 256 * 6;
+    const size_t smem = static_cast<size_t>(threads) * kObSmallItems * 12 + static_cast<size_t>(threads / 32) * 256 * 6;
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(ob_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(ob_small_kernel)");

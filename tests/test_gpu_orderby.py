@@ -134,3 +134,16 @@ def test_order_by_forms_and_skipped_digits(cuda, n, shape):
         ob.OrderByColumn(None, _dev(cols[i]), None if not nulls or nulls[i] is None else _dev(nulls[i].view(np.int64)),
                          n, int(desc[i]))
     assert (ob.indices[:n].cpu().numpy() == exp).all()
+
+
+@pytest.mark.parametrize("n", [200, 9000])
+def test_order_by_column_of_chosen_rows(cuda, n):
+    """OrderByColumn over row numbers of a longer column (first == 0): both forms keep them whole."""
+    from qikkdb_b200 import _capi as capi
+    rng = np.random.default_rng(n)
+    col = rng.integers(-50, 50, 300_000).astype(np.int32)
+    rows = rng.permutation(len(col))[:n].astype(np.int32)
+    idx, dc = _dev(rows), _dev(col)
+    capi.check(capi.lib().qdb_order_by_column(capi.QDB_INT32, dc.data_ptr(), None, 0, n, 0, idx.data_ptr(),
+                                              torch.cuda.current_stream().cuda_stream))
+    assert (idx.cpu().numpy() == rows[np.argsort(col[rows], kind="stable")]).all()
