@@ -1319,10 +1319,9 @@ template <typename KT, bool COMP, typename VT, typename PT, bool NULLS>
 int32_t launch_agg_t(const AggArgs& a, size_t smem, cudaStream_t st) {
     auto kern = gb_agg_kernel<KT, COMP, VT, PT, NULLS>;
     const DeviceInfo& di = device_info();
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gb_agg_kernel)");
-    }
+    static std::atomic<uint64_t> allowed{0};
+    const int32_t rc = allow_dynamic_smem(reinterpret_cast<const void*>(kern), allowed, "gb_agg_kernel shared memory");
+    if (rc != QDB_OK) return rc;
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kAggThreads, smem);
     if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
@@ -1345,10 +1344,9 @@ int32_t launch_agg_t(const AggArgs& a, size_t smem, cudaStream_t st) {
 template <typename VT>
 int32_t launch_spill_t(const AggArgs& a, size_t smem, int64_t grid, cudaStream_t st) {
     auto kern = gb_spill_kernel<VT>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gb_spill_kernel)");
-    }
+    static std::atomic<uint64_t> allowed{0};
+    const int32_t rc = allow_dynamic_smem(reinterpret_cast<const void*>(kern), allowed, "gb_spill_kernel shared memory");
+    if (rc != QDB_OK) return rc;
     kern<<<static_cast<unsigned>(grid), kSpillThreads, smem, st>>>(a);
     note_launch();
     cudaError_t e = cudaGetLastError();

@@ -1311,8 +1311,9 @@ template <typename KT, bool COMP, typename VT, typename PT, int MODE>
 int32_t launch_fast_t(const AggArgs& a, size_t smem, cudaStream_t st) {
     auto kern = gb_fast_kernel<KT, COMP, VT, PT, MODE>;
     const DeviceInfo& di = device_info();
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gb_fast_kernel)");
+    static std::atomic<uint64_t> allowed{0};
+    const int32_t rc = allow_dynamic_smem(reinterpret_cast<const void*>(kern), allowed, "gb_fast_kernel shared memory");
+    if (rc != QDB_OK) return rc;
     int64_t grid = std::min<int64_t>(di.sm_count, a.tiles);
     if (a.spill_keys) {
         if (a.spill_ctas > grid) return fail(QDB_ERROR, "gb_fast_kernel: spill plan needs more CTAs than fit");
@@ -1321,7 +1322,7 @@ int32_t launch_fast_t(const AggArgs& a, size_t smem, cudaStream_t st) {
     if (grid < 1) return QDB_OK;
     kern<<<static_cast<unsigned>(grid), kFastThreads, smem, st>>>(a);
     note_launch();
-    e = cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "gb_fast_kernel launch");
     return QDB_OK;
 }
@@ -1329,10 +1330,9 @@ int32_t launch_fast_t(const AggArgs& a, size_t smem, cudaStream_t st) {
 template <typename VT, int MODE>
 int32_t launch_fspill_t(const AggArgs& a, size_t smem, int64_t grid, int32_t slices, cudaStream_t st) {
     auto kern = gb_fspill_kernel<VT, MODE>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gb_fspill_kernel)");
-    }
+    static std::atomic<uint64_t> allowed{0};
+    const int32_t rc = allow_dynamic_smem(reinterpret_cast<const void*>(kern), allowed, "gb_fspill_kernel shared memory");
+    if (rc != QDB_OK) return rc;
     kern<<<static_cast<unsigned>(grid), kFSpillThreads<MODE>, smem, st>>>(a, slices);
     note_launch();
     cudaError_t e = cudaGetLastError();

@@ -130,11 +130,12 @@ __global__ void __launch_bounds__(kFewThreads, 1) gb_few_kernel(const AggArgs a)
 template <typename KT, bool COMP, typename VT, int MODE>
 int32_t launch_few_t(const AggArgs& a, size_t smem, int64_t grid, cudaStream_t st) {
     auto kern = gb_few_kernel<KT, COMP, VT, MODE>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gb_few_kernel)");
+    static std::atomic<uint64_t> allowed{0};
+    const int32_t rc = allow_dynamic_smem(reinterpret_cast<const void*>(kern), allowed, "gb_few_kernel shared memory");
+    if (rc != QDB_OK) return rc;
     kern<<<static_cast<unsigned>(grid), kFewThreads, smem, st>>>(a);
     note_launch();
-    e = cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? QDB_OK : cuda_fail(e, "gb_few_kernel launch");
 }
 

@@ -541,11 +541,14 @@ static int32_t ob_column(const void* col, const uint64_t* nulls, int32_t desc, i
     using K = typename std::conditional<sizeof(T) == 4, uint32_t, uint64_t>::type;
     constexpr int D = sizeof(K);
     const int64_t tiles = (n + kObTile<K> - 1) / kObTile<K>;
+    static std::atomic<uint64_t> allowed{0};
+    int32_t rc = allow_dynamic_smem(reinterpret_cast<const void*>(ob_pass_kernel<K>), allowed, "ob_pass_kernel shared memory");
+    if (rc != QDB_OK) return rc;
     // One allocation: the digit counts, the passes and the tile states (cleared), two key and two row buffers.
     const size_t hist_b = D * 256 * sizeof(uint32_t), pass_b = 256, state_b = static_cast<size_t>(tiles) * 256 * 8;
     const size_t key_b = (static_cast<size_t>(n) * sizeof(K) + 255) / 256 * 256, idx_b = (static_cast<size_t>(n) * 4 + 255) / 256 * 256;
     unsigned char* mem = nullptr;
-    int32_t rc = dev_alloc(reinterpret_cast<void**>(&mem), hist_b + pass_b + state_b + 2 * key_b + 2 * idx_b, s);
+    rc = dev_alloc(reinterpret_cast<void**>(&mem), hist_b + pass_b + state_b + 2 * key_b + 2 * idx_b, s);
     if (rc != QDB_OK) return rc;
     ObArgs<K> a;
     uint32_t* hist = reinterpret_cast<uint32_t*>(mem);
@@ -561,8 +564,7 @@ static int32_t ob_column(const void* col, const uint64_t* nulls, int32_t desc, i
     a.n = n;
     a.first = first ? 1 : 0;
     constexpr size_t smem = static_cast<size_t>(kObTile<K>) * (sizeof(K) + 4) + kObWarps * 256 * 6;
-    cudaError_t e = cudaFuncSetAttribute(ob_pass_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e == cudaSuccess) e = cudaMemsetAsync(mem, 0, hist_b + pass_b + state_b, s);
+    cudaError_t e = cudaMemsetAsync(mem, 0, hist_b + pass_b + state_b, s);
     if (e == cudaSuccess) {
         const DeviceInfo& di = device_info();
         const unsigned g = static_cast<unsigned>(std::min<int64_t>((n + kObThreads - 1) / kObThreads, int64_t(di.sm_count) * 4));
@@ -581,10 +583,9 @@ static int32_t ob_small(const ObSmallArgs& a, cudaStream_t s) {
     const int per = 32 * kObSmallItems;
     const int threads = std::max(4, (a.n + per - 1) / per) * 32;  // at least four warps share the digit scans
     const size_t smem = static_cast<size_t>(threads) * kObSmallItems * 12 + static_cast<size_t>(threads / 32) * 256 * 6;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(ob_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(ob_small_kernel)");
-    }
+    static std::atomic<uint64_t> allowed{0};
+    const int32_t rc = allow_dynamic_smem(reinterpret_cast<const void*>(ob_small_kernel), allowed, "ob_small_kernel shared memory");
+    if (rc != QDB_OK) return rc;
     ob_small_kernel<<<1, threads, smem, s>>>(a);
     note_launch();
     const cudaError_t e = cudaGetLastError();

@@ -2,6 +2,7 @@
 // hashing, value encodings and streaming loads.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <cstring>
 #include <type_traits>
@@ -37,6 +38,11 @@ const DeviceInfo& device_info();
 
 // Counts this library's kernel launches (reported by qdb_launch_count()).
 void note_launch(int64_t n = 1);
+
+// Lets `kernel` be launched with as much dynamic shared memory as the current device has, once per kernel and device
+// (`done`: one per kernel, a bit per device).  The limit belongs to the process, not to a call: a call that set it to its
+// own size would make the launch of another thread fail whose larger size was set just before.
+int32_t allow_dynamic_smem(const void* kernel, std::atomic<uint64_t>& done, const char* name);
 
 // Stream-ordered allocation helpers (the pool keeps freed blocks for reuse).
 int32_t dev_alloc(void** p, size_t bytes, cudaStream_t s);

@@ -57,6 +57,20 @@ const DeviceInfo& device_info() {
     return di;
 }
 
+int32_t allow_dynamic_smem(const void* kernel, std::atomic<uint64_t>& done, const char* name) {
+    const DeviceInfo& di = device_info();
+    const uint64_t bit = di.device >= 0 && di.device < 64 ? uint64_t(1) << di.device : 0;
+    if (done.load(std::memory_order_acquire) & bit) return QDB_OK;
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 di.max_smem_optin - static_cast<int>(fa.sharedSizeBytes));
+    if (e != cudaSuccess) return cuda_fail(e, name);
+    done.fetch_or(bit, std::memory_order_release);
+    return QDB_OK;
+}
+
 int32_t dev_alloc(void** p, size_t bytes, cudaStream_t s) {
     *p = nullptr;
     if (bytes == 0) return QDB_OK;
