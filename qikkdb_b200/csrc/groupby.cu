@@ -371,7 +371,7 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
     if (a.nul) {
         a.ptype = ptype;
         a.null_keys = a.knull0 != nullptr;
-        a.wide = vk == VK_F64 && a.has_sum;
+        a.wide = (vk == VK_F32 || vk == VK_F64) && a.has_sum;
     }
     // Stages: enough bytes in flight to cover the HBM latency at an SM's share of the bandwidth (about 48 KB), and at
     // least three when they fit (a warp may hold two stages while it carries rows over).

@@ -101,7 +101,7 @@ struct AggArgs {
     int32_t fits = 0;      // 1: every group fits the table: a key may overflow into the next probe_b - 1 buckets
     int32_t probe_b = 1;   // buckets a claim may visit
     // Calls of the fast pass with NULL masks or a row mask: the predicate's type (0 none), whether a key may be NULL, sums
-    // of doubles in 96 bits (a third limb at so_l2), and the warps' queues of keys to look up.
+    // of floats and doubles in 96 bits (a third limb at so_l2), and the warps' queues of keys to look up.
     int32_t nul = 0;
     int32_t ptype = 0;
     int32_t null_keys = 0;

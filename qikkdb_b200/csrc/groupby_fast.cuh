@@ -134,8 +134,13 @@ static __device__ __noinline__ int fclaim(const FTab t, uint32_t b, uint64_t kw,
 // (|v| < 2^emax) of the CTA's first tile; values up to 2^(emax + 2) are kept.
 //   float: q = m24 << sh with sh = biased exponent - sh0 in [0, 39 - hb]: exact.
 //   double: q = round(v * 2^F) for |v| in [lo, hi): every kept value has at least 24 significant bits.
-// FM_WIDE keeps doubles in 96 bits (three limbs), so that addends need no headroom: q = round(v * 2^(61 - emax)) for |v|
-// below 2^(emax + 2), every bit of a value down to 2^(emax - 9) and at least 40 bits of any kept one.
+// FM_WIDE (calls with NULL masks or a row mask) keeps sums in 96 bits (three limbs), so that 64-bit addends need no
+// headroom and the window is wide enough for columns that grow along their rows: values up to 2^(emax + 15) and down to
+// 2^(emax - 24) are kept.  (With the 2^(emax + 2) of the 64-bit sums, 2^23 masked rows that grow 2^12-fold over 10 groups
+// took 7.3 ms in FP64 atomics on ten words, 0.11 ms in the general pass.)
+//   float: q = m24 << sh with sh in [0, 38]: exact.
+//   double: q = round(v * 2^F) for |v| < 2^(emax + 2) and round(v * 2^(F - 13)) << 13 above, F = 61 - emax, less for CTAs
+//   of 2^19 rows and more so that 2^hb values of 2^(emax + 15) fit 96 bits: at least 37 bits of any kept value.
 // ---------------------------------------------------------------------------------------------
 struct FixQ {
     int sh0 = 0;
@@ -144,19 +149,29 @@ struct FixQ {
     double inv = 1.0;    // 2^-F
     double lo = 0.0;
     double hi = 0.0;
+    double top = 0.0;        // FM_WIDE doubles: values in [hi, top) are added kWideShift bits up
 };
+constexpr int kWideShift = 13;
 
 template <typename VT, bool WIDE>
 __device__ __forceinline__ FixQ fixq(int emax, int hb) {
     FixQ f;
-    emax = max(-900, min(900, emax));
-    if constexpr (WIDE) {
-        f.scale = ldexp(1.0, 61 - emax);
-        f.inv = ldexp(1.0, emax - 61);
-        f.lo = ldexp(1.0, emax - 22);
+    if constexpr (WIDE && std::is_same<VT, float>::value) {
+        f.shmax = 38;
+        f.sh0 = max(1, min(254 - f.shmax, emax + 103));  // 2^(emax + 14) <= |v| < 2^(emax + 15) takes sh = 38
+        f.inv = ldexp(1.0, f.sh0 - 150);
+        return f;
+    } else if constexpr (WIDE) {
+        emax = max(-960, min(960, emax));
+        const int F = 61 - emax - max(0, hb - 19);
+        f.scale = ldexp(1.0, F);
+        f.inv = ldexp(1.0, -F);
+        f.lo = ldexp(1.0, emax - 24);
         f.hi = ldexp(1.0, emax + 2);
+        f.top = ldexp(1.0, emax + 2 + kWideShift);
         return f;
     }
+    emax = max(-900, min(900, emax));
     const int g = 2;
     f.shmax = max(0, min(30, 39 - hb));
     if constexpr (std::is_same<VT, float>::value) {
@@ -175,7 +190,7 @@ __device__ __forceinline__ FixQ fixq(int emax, int hb) {
     return f;
 }
 
-template <typename VT>
+template <typename VT, bool WIDE>
 __device__ __forceinline__ long long addq(VT v, const FixQ& f, bool& ok) {
     if constexpr (std::is_same<VT, float>::value) {
         const uint32_t b = __float_as_uint(v);
@@ -184,12 +199,14 @@ __device__ __forceinline__ long long addq(VT v, const FixQ& f, bool& ok) {
         ok = inw | ((b << 1) == 0u);  // zero is exact; subnormals, NaN and Inf take the FP64 path
         const int32_t sg = static_cast<int32_t>(b) >> 31;
         const int32_t m = static_cast<int32_t>(((b & 0x7fffffu) | 0x800000u) ^ static_cast<uint32_t>(sg)) - sg;
-        // one widening multiply shifts and sign-extends (sh is at most shmax <= 30: hb is at least 9)
+        if constexpr (WIDE) return static_cast<long long>(inw ? m : 0) << (sh & 63u);
+        // one widening multiply shifts and sign-extends (fixq keeps sh at 30 or less)
         return static_cast<long long>(inw ? m : 0) * static_cast<long long>(static_cast<int32_t>(1u << (sh & 31u)));
     } else if constexpr (std::is_same<VT, double>::value) {
         const double m = fabs(v);
-        ok = (m == 0.0) | ((m >= f.lo) & (m < f.hi));  // false for NaN and Inf
-        return ok ? __double2ll_rn(v * f.scale) : 0ll;
+        ok = (m == 0.0) | ((m >= f.lo) & (m < (WIDE ? f.top : f.hi)));  // false for NaN and Inf
+        const double down = WIDE && m >= f.hi ? 1.0 / (1 << kWideShift) : 1.0;  // update() shifts the addend back up
+        return ok ? __double2ll_rn(v * down * f.scale) : 0ll;
     } else {
         ok = true;
         return static_cast<long long>(v);
@@ -338,7 +355,7 @@ constexpr int FM_MM = 2;
 constexpr int FM_VALS = 4;
 constexpr int FM_KZ = 8;  // the key column is an AAFL-compressed block (single key, not DOUBLE)
 constexpr int FM_NULL = 32;  // NULL masks (key, value, predicate) or a row mask; the predicate type is read at run time
-constexpr int FM_WIDE = 64;  // 96-bit sums of doubles
+constexpr int FM_WIDE = 64;  // 96-bit sums of floats and doubles
 constexpr int FM_KMOD = 16;  // keys are replaced by key % m as they are read (single INT32 or INT64 key)
 
 // K32: every key word is a 32-bit key's, so none equals kEmpty.
@@ -414,7 +431,14 @@ struct FastWarp {
         const uint32_t o = s << t.osh;
         reds_add(t.cnt + o, 1u);
         if constexpr (SUM) {
-            const unsigned long long uq = static_cast<unsigned long long>(q);
+            unsigned long long uq = static_cast<unsigned long long>(q);
+            unsigned x2 = q < 0 ? 0xffffffffu : 0u;  // the addend's third word (FM_WIDE)
+            if constexpr (WIDE && std::is_same<VT, double>::value) {
+                if (fabs(v) >= fq.hi) {
+                    x2 = static_cast<unsigned>(q >> (64 - kWideShift));
+                    uq <<= kWideShift;
+                }
+            }
             const unsigned x0 = static_cast<unsigned>(uq);
             const unsigned old0 = atoms_add(t.l0 + o, x0);
             const unsigned c = (old0 + x0 < old0) ? 1u : 0u;
@@ -422,7 +446,7 @@ struct FastWarp {
                 const unsigned long long y1 = (uq >> 32) + c;
                 const unsigned x1 = static_cast<unsigned>(y1);
                 const unsigned old1 = atoms_add(t.l1 + o, x1);
-                const unsigned y2 = (q < 0 ? 0xffffffffu : 0u) + static_cast<unsigned>(y1 >> 32) + ((old1 + x1 < old1) ? 1u : 0u);
+                const unsigned y2 = x2 + static_cast<unsigned>(y1 >> 32) + ((old1 + x1 < old1) ? 1u : 0u);
                 if (y2) reds_add(t.l2 + o, y2);
             } else {
                 reds_add(t.l1 + o, static_cast<unsigned>(uq >> 32) + c);
@@ -473,7 +497,7 @@ struct FastWarp {
         for (int u = 0; u < U; ++u) {
             look[u] = true;
             q[u] = 0;
-            if constexpr (SUM) q[u] = addq<VT>(v[u], fq, look[u]);
+            if constexpr (SUM) q[u] = addq<VT, WIDE>(v[u], fq, look[u]);
             look[u] = look[u] & act[u];
             if constexpr (!K32) look[u] = look[u] & (kw[u] != kEmpty);
             m[u] = fhash(kw[u]);
@@ -526,7 +550,7 @@ struct FastWarp {
         for (int u = 0; u < U; ++u) {
             inwin[u] = true;
             q[u] = 0;
-            if constexpr (SUM) q[u] = addq<VT>(v[u], fq, inwin[u]);
+            if constexpr (SUM) q[u] = addq<VT, WIDE>(v[u], fq, inwin[u]);
             if constexpr (NUL) inwin[u] = inwin[u] | vn[u];
             m[u] = fhash(kw[u]);
             look[u] = act[u] & (kw[u] != kEmpty) & inwin[u] & use_smem;
@@ -1375,7 +1399,7 @@ int32_t launch_fast_m(const AggArgs& a, size_t smem, cudaStream_t st) {
 // Calls with NULL masks or a row mask (single key): one instantiation per key type, value type and aggregate set.
 template <typename KT, typename VT, int MODE>
 int32_t launch_fast_nul_t(const AggArgs& a, size_t smem, cudaStream_t st) {
-    constexpr int W = (std::is_same<VT, double>::value && (MODE & FM_SUM)) ? FM_WIDE : 0;
+    constexpr int W = (std::is_floating_point<VT>::value && (MODE & FM_SUM)) ? FM_WIDE : 0;
     return launch_fast_t<KT, false, VT, NoPred, MODE | FM_NULL | W>(a, smem, st);
 }
 
@@ -1427,7 +1451,7 @@ int32_t launch_fast_k(const AggArgs& a, ValKind vk, int32_t ptype, size_t smem, 
 
 template <typename VT>
 int32_t launch_fspill_m(const AggArgs& a, size_t smem, int64_t grid, int32_t slices, cudaStream_t st) {
-    if constexpr (std::is_same<VT, double>::value) {
+    if constexpr (std::is_floating_point<VT>::value) {
         if (a.wide && fast_mode(a) == (FM_VALS | FM_SUM))
             return launch_fspill_t<VT, FM_VALS | FM_SUM | FM_WIDE>(a, smem, grid, slices, st);
         if (a.wide && fast_mode(a) == (FM_VALS | FM_SUM | FM_MM))

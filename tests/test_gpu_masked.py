@@ -3,10 +3,11 @@ at the edges of its 2048-row tile, tables that hold every group and tables that 
 or the empty slot's word, groups without a non-NULL value, and the accuracy of SUM and AVG of doubles."""
 import numpy as np
 import pytest
+import torch
 
 from gpu_compare import FLOAT_RTOL
-from qikkdb_b200.groupby import FilterConditions
-from test_gpu_parity import ALL, run_both
+from qikkdb_b200.groupby import FilterConditions, GroupByTable, device_nullmask
+from test_gpu_parity import ALL, _dev, run_both
 
 pytestmark = pytest.mark.gpu
 
@@ -93,3 +94,71 @@ def test_evenly_spaced_keys(cuda, groups, stride):
         k = rng.integers(0, groups, n).astype(np.int64) * np.int64(stride)
     run_both(k, rng.integers(-1000, 1000, n).astype(np.int32), ALL, groups)
     run_both(k, np.exp(rng.standard_normal(n)).astype(np.float32), ["sum", "max"], groups, val_is_float=True)
+
+
+def _growing(n, groups, dt, rng):
+    """A column whose first tiles hold values of about 1 and whose later rows, two by two in one group, hold v and its
+    negative, v up to 2^14, beside values of about 2^-22: every group's sum is a sum of the small ones alone.  All
+    values are multiples of 2^-46 and exact in either type."""
+    k = np.repeat(rng.integers(0, groups, (n + 3) // 4), 4)[:n].astype(np.int32)
+    v = np.empty(n, dtype=np.float64)
+    first = 148 * 2048
+    quad = np.arange(n) % 4
+    size = np.exp2(rng.integers(2, 14, (n + 3) // 4).astype(np.float64)).repeat(4)[:n]
+    size *= (1 + rng.integers(0, 1 << 23, (n + 3) // 4) / (1 << 23)).repeat(4)[:n]
+    small = (1 + rng.integers(0, 1 << 23, n) / (1 << 23)) * 2.0 ** -23
+    v = np.where(quad == 0, size, np.where(quad == 1, -size, small))
+    head = (1 + rng.integers(0, 1 << 20, (n + 3) // 4) / (1 << 20)).repeat(4)[:n]
+    head = np.where(quad % 2 == 0, head, -head)
+    v[:first] = head[:first]
+    return k, v.astype(dt)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("groups", [10, 2000])
+def test_masked_sums_of_growing_columns(cuda, groups, dt):
+    """Values far above and below those of a CTA's first tile (2^15 times up, 2^-23 down) stay in the 96-bit sums, which
+    are exact here, whatever the order: a row added in FP64 instead would leave its rounding at 2^14's last place."""
+    n = 1_600_000
+    rng = np.random.default_rng(groups)
+    k, v = _growing(n, groups, dt, rng)
+    vn = np.zeros(n, bool)
+    vn[rng.integers(148 * 2048 // 4, n // 4, n // 50) * 4 + 2] = True  # small ones: sums stay below 2^53 units of 2^-46
+    t = GroupByTable(["sum"], np.int32, dt, groups)
+    t.process([_dev(k)], _dev(v), n, None, device_nullmask(vn))
+    r = t.results_numpy()
+    ints = np.where(vn, 0, np.round(v.astype(np.float64) * 2.0 ** 46)).astype(np.int64)  # exact: below 2^61
+    exp = np.zeros(groups, dtype=np.int64)
+    np.add.at(exp, k, ints)
+    order = np.argsort(r["keys"][0])
+    keys = r["keys"][0][order]
+    assert len(keys) == len(np.unique(k))
+    assert (r["sum"][order] == (exp[keys].astype(np.float64) * 2.0 ** -46).astype(dt)).all()
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_masked_growing_column_stays_on_chip(cuda, monkeypatch, dt):
+    """A column that grows 2^12-fold along its rows, 10 groups: no slower than the general pass (rows that leave the
+    fixed-point window would be added to ten words of the global table)."""
+    n = 1 << 23
+    g = torch.Generator(device="cuda").manual_seed(1)
+    k = torch.randint(0, 10, (n,), generator=g, device="cuda", dtype=torch.int32)
+    tt = torch.float32 if dt == np.float32 else torch.float64
+    v = torch.rand(n, generator=g, device="cuda", dtype=tt) + torch.arange(n, device="cuda", dtype=tt) * (4096.0 / n)
+    null = torch.zeros(n // 64, dtype=torch.int64, device="cuda")
+    null[::3] = 5
+    t = GroupByTable(["sum"], np.int32, dt, 10)
+    us = {}
+    for fast in ("1", "0"):
+        monkeypatch.setenv("QDB_AGG_FAST", fast)
+        best = float("inf")
+        for _ in range(4):
+            t.reset()
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            t.process([k], v, n, None, null, sync=False)
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]) * 1e3)
+        us[fast] = best
+    assert us["1"] <= us["0"], us
