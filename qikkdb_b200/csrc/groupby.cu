@@ -128,9 +128,7 @@ static int32_t launch_few(const qdb_gb* gb, const AggArgs& a, size_t smem, int64
     if (gb->n_key_cols == 2) return launch_few_comp(a, vk, smem, grid, st);
     switch (gb->key_type) {
         case QDB_INT32: return launch_few_i32(a, vk, smem, grid, st);
-        case QDB_INT64: return launch_few_i64(a, vk, smem, grid, st);
         case QDB_FLOAT: return launch_few_f32(a, vk, smem, grid, st);
-        case QDB_DOUBLE: return launch_few_f64(a, vk, smem, grid, st);
         default: return fail(QDB_ERR_INVALID, "unsupported key type");
     }
 }
@@ -443,8 +441,9 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
     };
 
     // A table that holds every group at half load or less (a quarter when it can) takes the pass without a ring, where the
-    // whole of shared memory is the table: a CTA per SM, or as many as there are steps of rows.
-    if (!a.nul && !a.kz) {
+    // whole of shared memory is the table: a CTA per SM, or as many as there are steps of rows.  Rows of 4-byte keys and
+    // values that all count only: predicates and wider rows are faster staged (groupby_few.cuh has both sides).
+    if (!a.nul && !a.kz && !a.pcol && ks == 4 && vs <= 4) {
         const size_t bytes = static_cast<size_t>(di.max_smem_optin) - 1024;
         const uint64_t groups = static_cast<uint64_t>(gb->capacity) + 1;
         uint64_t most = bytes / bucket_bytes;
@@ -457,7 +456,6 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
             a.fits = 1;
             a.probe_b = std::min(kProbeBuckets, NB);
             a.flush_rounds = static_cast<int32_t>(env_int("QDB_FLUSH_ROUNDS", 16));
-            a.ptype = ptype;
             *used = true;
             return launch_few(gb, a, smem, grid, s);
         }

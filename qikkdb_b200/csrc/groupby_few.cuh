@@ -1,5 +1,5 @@
-// The aggregation pass of a table that holds every group (few groups: nothing spills), for calls without NULL masks, a
-// row mask or compressed keys.
+// The aggregation pass of a table that holds every group (few groups: nothing spills), for calls over 4-byte keys (or two
+// of them) and 4-byte values in which every row counts: no predicate, NULL masks, row mask or compressed keys.
 //
 // The staged pass (groupby_fast.cuh) keeps one CTA of 16 consumer warps per SM fed through a ring of tiles, with lists of
 // passing rows, stages carried over and spill bookkeeping: 124 warp instructions per 32 rows, issued by 4.25 warps per
@@ -8,6 +8,11 @@
 // to the table, and the shared memory the ring took holds twice as many groups.  It is bound by its instructions.
 // 2^27 rows over 10 groups (int32 keys, float values, AVG and COUNT): 662 us staged, 503 us here; 2^26 rows over 2000
 // groups, SUM/MIN/MAX/COUNT of int32: 483 and 377 us.
+//
+// Other calls are faster staged.  A predicate's list leaves the table's instructions to the passing rows: 2^24 rows over
+// 300 groups (int64 keys, SUM/MIN/MAX/COUNT of double) at 5 % take 100 us staged and 206 us in a form of this pass with
+// predicates.  Rows of 12 and 16 bytes leave registers for two of them a thread: 2^26 rows of int64 keys and values, SUM
+// over 1000 groups, 323 us staged and 531 us.
 #pragma once
 
 #include "groupby_fast.cuh"
@@ -19,17 +24,14 @@ constexpr int kFewThreads = 768;  // 24 warps, 80 registers
 template <typename T, int U>
 __device__ __forceinline__ void few_load(const void* col, int64_t r, int64_t n, T (&out)[U]) {
     const T* p = static_cast<const T*>(col) + r;
-    constexpr int kBytes = static_cast<int>(sizeof(T)) * U;
+    static_assert(sizeof(T) == 4 && (U == 2 || U == 4), "one 8- or 16-byte load");
     if (r + U <= n) {
-        if constexpr (kBytes == 8) {
+        if constexpr (U == 2) {
             const int2 q = __ldcs(reinterpret_cast<const int2*>(p));
             memcpy(out, &q, 8);
         } else {
-#pragma unroll
-            for (int i = 0; i < kBytes / 16; ++i) {
-                const int4 q = __ldcs(reinterpret_cast<const int4*>(p) + i);
-                memcpy(reinterpret_cast<char*>(out) + 16 * i, &q, 16);
-            }
+            const int4 q = __ldcs(reinterpret_cast<const int4*>(p));
+            memcpy(out, &q, 16);
         }
     } else {
 #pragma unroll
@@ -37,7 +39,7 @@ __device__ __forceinline__ void few_load(const void* col, int64_t r, int64_t n, 
     }
 }
 
-// KT, COMP, VT, MODE as gb_fast_kernel's; the predicate's type is read at run time.
+// KT, COMP, VT, MODE as gb_fast_kernel's.
 template <typename KT, bool COMP, typename VT, int MODE>
 __global__ void __launch_bounds__(kFewThreads, 1) gb_few_kernel(const AggArgs a) {
     extern __shared__ __align__(128) unsigned char sm[];
@@ -46,8 +48,8 @@ __global__ void __launch_bounds__(kFewThreads, 1) gb_few_kernel(const AggArgs a)
     constexpr bool VFLOAT = std::is_floating_point<VT>::value;
     constexpr bool VALS = (MODE & FM_VALS) != 0;
     constexpr bool WIDE = false;
-    // Rows per thread and step: four where a row's key and value take 8 bytes, two of wider rows (registers).
-    constexpr int U = (!COMP && sizeof(KT) == 4 && sizeof(VT) == 4) ? 4 : 2;
+    // Rows per thread and step: four, two of composite keys (registers).
+    constexpr int U = COMP ? 2 : 4;
     const int lane = threadIdx.x & 31;
 
     ftab_init<VT, WIDE>(sm, a, threadIdx.x, blockDim.x);
@@ -59,28 +61,10 @@ __global__ void __launch_bounds__(kFewThreads, 1) gb_few_kernel(const AggArgs a)
     int64_t r = (static_cast<int64_t>(blockIdx.x) * kFewThreads + threadIdx.x) * U;
     KT k0[U], k1[U];
     VT v[U];
-    uint64_t p[U];  // raw predicate values
     auto load = [&](int64_t at) {
         few_load(a.key0, at, a.n, k0);
         if constexpr (COMP) few_load(a.key1, at, a.n, k1);
         if constexpr (VALS) few_load(a.vals, at, a.n, v);
-        if (pred_size(a.ptype) == 4) {
-            uint32_t w[U];
-            few_load(a.pcol, at, a.n, w);
-#pragma unroll
-            for (int u = 0; u < U; ++u) p[u] = w[u];
-        } else if (a.ptype) {
-            few_load(a.pcol, at, a.n, p);
-        }
-    };
-    auto passes = [&](uint64_t x) -> bool {
-        switch (a.ptype) {
-            case QDB_INT32: return pred_pass<int32_t>(a.pi, static_cast<int32_t>(x));
-            case QDB_INT64: return pred_pass<int64_t>(a.pi, static_cast<int64_t>(x));
-            case QDB_FLOAT: return pred_pass<float>(a.pi, __uint_as_float(static_cast<uint32_t>(x)));
-            case QDB_DOUBLE: return pred_pass<double>(a.pi, __longlong_as_double(static_cast<long long>(x)));
-            default: return true;
-        }
     };
     load(r);
     __syncthreads();
@@ -108,7 +92,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) gb_few_kernel(const AggArgs a)
         VT cv[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            act[u] = r + u < a.n && passes(p[u]);
+            act[u] = r + u < a.n;
             if constexpr (COMP) kw[u] = composite_word(static_cast<int32_t>(k0[u]), static_cast<int32_t>(k1[u]));
             else kw[u] = key_word(k0[u]);
             if constexpr (!COMP && std::is_integral<KT>::value) {
@@ -154,9 +138,7 @@ int32_t launch_few_k(const AggArgs& a, ValKind vk, size_t smem, int64_t grid, cu
     if (fast_mode(a) == 0) return launch_few_t<KT, COMP, int32_t, 0>(a, smem, grid, st);
     switch (vk) {
         case VK_I32: return launch_few_m<KT, COMP, int32_t>(a, smem, grid, st);
-        case VK_I64: return launch_few_m<KT, COMP, int64_t>(a, smem, grid, st);
         case VK_F32: return launch_few_m<KT, COMP, float>(a, smem, grid, st);
-        case VK_F64: return launch_few_m<KT, COMP, double>(a, smem, grid, st);
         default: return fail(QDB_ERR_INVALID, "unsupported value type");
     }
 }
