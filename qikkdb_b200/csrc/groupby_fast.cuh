@@ -86,16 +86,23 @@ __device__ __forceinline__ FTab ftab(unsigned char* sm, const AggArgs& a) {
 // a partition's rows spread over every bucket of the spill pass's table), and bits 32..46 the bit of the seen-once
 // filter.  The global table hashes with the independent mix64.  Being linear it spreads dense and evenly spaced keys
 // better than chance (no full buckets at half load, against 7-10 % with a mixing hash, which made the spill pass of
-// 16.8M composite groups 4.2 instead of 3.8 ms), at the price of strides that it lines up: see falt.
+// 16.8M composite groups 4.2 instead of 3.8 ms), at the price of strides that it lines up: see ffar.
 __device__ __forceinline__ uint64_t fhash(uint64_t kw) { return kw * kHashMul; }
 __device__ __forceinline__ uint32_t fbucket(uint64_t m, int shift, uint32_t NB) {
     const uint32_t x = __funnelshift_rc(static_cast<uint32_t>(m), static_cast<uint32_t>(m >> 32), shift);
     return __umulhi(x, NB);
 }
 
-// The bucket a key whose home bucket is full tries next, from other bits of its hash: home buckets that an unlucky stride
-// of the keys lines up would also fill their neighbours.
-__device__ __forceinline__ uint32_t falt(uint64_t m, uint32_t NB) {
+// Where a key whose home bucket is full goes: to the home bucket's neighbour, which the linear hash leaves emptier than
+// chance, or to one from other bits of its hash, as home buckets that an unlucky stride of the keys lines up would also
+// fill their neighbours.  The first of them is looked into without a call; a key that is in neither it nor the home bucket
+// costs its warp a call in every step.  In the aggregation pass the first is the neighbour (2^26 rows, half selected, over
+// 300 float keys: 342 us, 512 with the far one first; over 3000 double keys 426 and 530), in the spill pass, whose
+// partitions an unlucky stride crowds, the far one (10M rows over 20,000 evenly spaced keys: 222 us, 763 with the
+// neighbour).  Looking into both inline costs registers that the passes do not have (33M masked rows of doubles: 1317
+// instead of 1235 us).
+__device__ __forceinline__ uint32_t fnext(uint32_t b, uint32_t NB) { return (b + 1u == NB) ? 0u : b + 1u; }
+__device__ __forceinline__ uint32_t ffar(uint64_t m, uint32_t NB) {
     return __umulhi((static_cast<uint32_t>(m) ^ static_cast<uint32_t>(m >> 32)) * 0x9E3779B1u, NB);
 }
 
@@ -107,12 +114,14 @@ __device__ __forceinline__ int fprobe(const FTab& t, uint32_t b, uint64_t kw, bo
     return (k0 == kw) ? static_cast<int>(b) : ((k1 == kw) ? static_cast<int>(t.NB + b) : -1);
 }
 
-// Finds or claims kw in bucket b, then in its second bucket and those after it (nb buckets in all): a new key is claimed
-// with a CAS on its key word.  Returns the slot or -1.
-static __device__ __noinline__ int fclaim(const FTab t, uint32_t b, uint64_t kw, int nb) {
+// Finds or claims kw in bucket b, then in the two that fnext and ffar give (far: in the second of them) and in those after
+// the far one (nb buckets in all): a new key is claimed with a CAS on its key word.  Returns the slot or -1.
+static __device__ __noinline__ int fclaim(const FTab t, uint32_t b, uint64_t kw, int nb, bool far) {
+    const uint32_t f = ffar(fhash(kw), t.NB);
     uint32_t bb = b;
     for (int k = 0; k < nb; ++k) {
-        if (k == 1) bb = falt(fhash(kw), t.NB);
+        if (k == 1 && !far) bb = fnext(b, t.NB);
+        else if (k == (far ? 1 : 2)) bb = f;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const uint32_t ka = t.keys + (bb * 2u + j) * 8u;
@@ -123,7 +132,7 @@ static __device__ __noinline__ int fclaim(const FTab t, uint32_t b, uint64_t kw,
                 if (prev == kEmpty || prev == kw) return static_cast<int>(j * t.NB + bb);
             }
         }
-        if (k) bb = (bb + 1u == t.NB) ? 0u : bb + 1u;
+        if (k > (far ? 0 : 1)) bb = fnext(bb, t.NB);
     }
     return -1;
 }
@@ -358,8 +367,8 @@ constexpr int FM_NULL = 32;  // NULL masks (key, value, predicate) or a row mask
 constexpr int FM_WIDE = 64;  // 96-bit sums of floats and doubles
 constexpr int FM_KMOD = 16;  // keys are replaced by key % m as they are read (single INT32 or INT64 key)
 
-// K32: every key word is a 32-bit key's, so none equals kEmpty.
-template <typename VT, int MODE, bool K32 = false>
+// K32: every key word is a 32-bit key's, so none equals kEmpty.  FAR: keys of a full home bucket go to the far one.
+template <typename VT, int MODE, bool K32 = false, bool FAR = false>
 struct FastWarp {
     static constexpr bool SUM = (MODE & FM_SUM) != 0;
     static constexpr bool MM = (MODE & FM_MM) != 0;
@@ -409,6 +418,12 @@ struct FastWarp {
             if (VALS) g_acc_row<VT>(slot, a, v);
             else g_count_row(slot, a.L);
         }
+    }
+
+    // Looks kw (hash m, home bucket b, full and without it) up in the next bucket it may be in: the slot or -1.
+    __device__ __forceinline__ int look_on(uint64_t kw, uint64_t m, uint32_t b) const {
+        bool empty;
+        return fprobe(t, FAR ? ffar(m, t.NB) : fnext(b, t.NB), kw, empty);
     }
 
     __device__ __forceinline__ void touch_queue(bool put, uint64_t kw, unsigned lane) {
@@ -519,9 +534,8 @@ struct FastWarp {
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 if (look[u] && !hit[u]) {
-                    bool e = false;
-                    int s2 = fprobe(t, falt(m[u], t.NB), kw[u], e);  // a key whose home bucket is full
-                    if (s2 < 0) s2 = fclaim(t, b[u], kw[u], probe_b);
+                    int s2 = look_on(kw[u], m[u], b[u]);  // a key whose home bucket is full
+                    if (s2 < 0) s2 = fclaim(t, b[u], kw[u], probe_b, FAR);
                     hit[u] = s2 >= 0;
                     slot[u] = static_cast<uint32_t>(s2);
                 }
@@ -577,8 +591,8 @@ struct FastWarp {
             }
         }
         if (fits) {
-            // A table sized for every group places a key whose home bucket is full in its second bucket, or rarely in one
-            // after it: look there before the claim path.
+            // A table sized for every group places a key whose home bucket is full in the next one, or rarely in one after
+            // it: look there before the claim path.
             bool nx[U], any_nx = false;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -589,8 +603,7 @@ struct FastWarp {
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     if (nx[u]) {
-                        bool e2 = false;
-                        const int s2 = fprobe(t, falt(m[u], t.NB), kw[u], e2);
+                        const int s2 = look_on(kw[u], m[u], b[u]);
                         if (s2 >= 0) {
                             slot[u] = s2;
                             hit[u] = true;
@@ -618,7 +631,7 @@ struct FastWarp {
                     go = (atoms_or(seen + (hb >> 5) * 4u, bit) & bit) != 0u;
                 }
                 if (go) {
-                    slot[u] = fclaim(t, b[u], kw[u], fits ? probe_b : 1);
+                    slot[u] = fclaim(t, b[u], kw[u], fits ? probe_b : 1, FAR);
                     hit[u] = slot[u] >= 0;
                 }
             }
@@ -818,7 +831,7 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
     __syncthreads();
     if constexpr (NUL) {
         if (a.null_keys && threadIdx.x == 0)  // an empty table always has room in the home bucket
-            s_null_slot = fclaim(tab, fbucket(fhash(kNullWord), 32, tab.NB), kNullWord, 1);
+            s_null_slot = fclaim(tab, fbucket(fhash(kNullWord), 32, tab.NB), kNullWord, 1, false);
         __syncthreads();
     }
 
@@ -1298,7 +1311,7 @@ __global__ void __launch_bounds__(kFSpillThreads<MODE>, 1) gb_fspill_kernel(cons
         __syncthreads();
         const int hb = max(1, 64 - __clzll(static_cast<long long>(total)));
         const FixQ fq = fixq<VT, WIDE>(s_emax == INT_MIN ? 0 : s_emax, hb);
-        FastWarp<VT, MODE> fw(a, tab, fq, &s_claims);
+        FastWarp<VT, MODE, false, true> fw(a, tab, fq, &s_claims);
         fw.bshift = 32 - a.spill_bits;
         fw.fits = a.fits != 0;
         fw.probe_b = a.probe_b;
