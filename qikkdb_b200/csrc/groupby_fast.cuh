@@ -93,14 +93,13 @@ __device__ __forceinline__ uint32_t fbucket(uint64_t m, int shift, uint32_t NB) 
     return __umulhi(x, NB);
 }
 
-// Where a key whose home bucket is full goes: to the home bucket's neighbour, which the linear hash leaves emptier than
-// chance, or to one from other bits of its hash, as home buckets that an unlucky stride of the keys lines up would also
-// fill their neighbours.  The first of them is looked into without a call; a key that is in neither it nor the home bucket
-// costs its warp a call in every step.  In the aggregation pass the first is the neighbour (2^26 rows, half selected, over
-// 300 float keys: 342 us, 512 with the far one first; over 3000 double keys 426 and 530), in the spill pass, whose
-// partitions an unlucky stride crowds, the far one (10M rows over 20,000 evenly spaced keys: 222 us, 763 with the
-// neighbour).  Looking into both inline costs registers that the passes do not have (33M masked rows of doubles: 1317
-// instead of 1235 us).
+// Where a key whose home bucket is full goes: to the two buckets behind it, which the linear hash leaves emptier than
+// chance, then to one from other bits of its hash, as home buckets that an unlucky stride of the keys lines up would also
+// fill their neighbours.  The next bucket is looked into without a call; a key beyond it costs its warp a call in every
+// step.  Both ends matter: with the far bucket first, 2^26 rows, half selected, over 300 float keys take 512 us (342 now),
+// and 2^24 rows over 30,000 keys spaced by 0x9E3779B1, SUM/MIN/MAX/COUNT, 277 us in the spill pass (190 now); without it
+// 10M rows over 20,000 keys spaced by 0x9E3779B97F4A7C15 take 763 us there.  Looking into two more buckets inline costs
+// registers that the passes do not have (33M masked rows of doubles: 1317 instead of 1235 us).
 __device__ __forceinline__ uint32_t fnext(uint32_t b, uint32_t NB) { return (b + 1u == NB) ? 0u : b + 1u; }
 __device__ __forceinline__ uint32_t ffar(uint64_t m, uint32_t NB) {
     return __umulhi((static_cast<uint32_t>(m) ^ static_cast<uint32_t>(m >> 32)) * 0x9E3779B1u, NB);
@@ -114,14 +113,12 @@ __device__ __forceinline__ int fprobe(const FTab& t, uint32_t b, uint64_t kw, bo
     return (k0 == kw) ? static_cast<int>(b) : ((k1 == kw) ? static_cast<int>(t.NB + b) : -1);
 }
 
-// Finds or claims kw in bucket b, then in the two that fnext and ffar give (far: in the second of them) and in those after
-// the far one (nb buckets in all): a new key is claimed with a CAS on its key word.  Returns the slot or -1.
-static __device__ __noinline__ int fclaim(const FTab t, uint32_t b, uint64_t kw, int nb, bool far) {
-    const uint32_t f = ffar(fhash(kw), t.NB);
-    uint32_t bb = b;
-    for (int k = 0; k < nb; ++k) {
-        if (k == 1 && !far) bb = fnext(b, t.NB);
-        else if (k == (far ? 1 : 2)) bb = f;
+// Finds or claims kw in bucket b, its two neighbours, the far one and those after it (nb buckets in all): a new key is
+// claimed with a CAS on its key word.  full: bucket b is full and without kw.  Returns the slot or -1.
+static __device__ __noinline__ int fclaim(const FTab t, uint32_t b, uint64_t kw, int nb, bool full) {
+    uint32_t bb = full ? fnext(b, t.NB) : b;
+    for (int k = full ? 1 : 0; k < nb; ++k) {
+        if (k == 3) bb = ffar(fhash(kw), t.NB);
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const uint32_t ka = t.keys + (bb * 2u + j) * 8u;
@@ -132,7 +129,7 @@ static __device__ __noinline__ int fclaim(const FTab t, uint32_t b, uint64_t kw,
                 if (prev == kEmpty || prev == kw) return static_cast<int>(j * t.NB + bb);
             }
         }
-        if (k > (far ? 0 : 1)) bb = fnext(bb, t.NB);
+        bb = fnext(bb, t.NB);
     }
     return -1;
 }
@@ -259,7 +256,8 @@ __device__ __forceinline__ void ftab_init(unsigned char* sm, const AggArgs& a, i
 // after a.flush_rounds rounds (a long probe run) finishes with the one-key search, which bounds the probe and reports
 // a full table.
 
-template <typename VT, bool WIDE>
+// SPILL: the table of a spill item, which has no copies of states and no NULL key.
+template <typename VT, bool WIDE, bool SPILL = false>
 __device__ __forceinline__ void ftab_flush(unsigned char* sm, const AggArgs& a, const FixQ& fq,
                                            unsigned long long* claims, bool null_seen = true) {
     constexpr bool V32 = sizeof(VT) == 4;
@@ -286,7 +284,7 @@ __device__ __forceinline__ void ftab_flush(unsigned char* sm, const AggArgs& a, 
             key[u] = (ki < S) ? keys[ki] : kEmpty;
             g[u] = nullptr;
             pend[u] = key[u] != kEmpty;
-            if (a.null_keys && key[u] == kNullWord) {
+            if (!SPILL && a.null_keys && key[u] == kNullWord) {
                 g[u] = null_seen ? g_special(a.main, W, 0, claims) : nullptr;
                 pend[u] = false;
             }
@@ -324,15 +322,16 @@ __device__ __forceinline__ void ftab_flush(unsigned char* sm, const AggArgs& a, 
             if (pend[u]) g[u] = g_find_from(a.main, W, key[u], pos[u], cur[u], a.counters, claims);
             if (!g[u]) continue;
             const int ki = i0 + u * blockDim.x;
-            const int i = ((ki & 1) * a.NB + (ki >> 1)) << a.rep_shift;  // key index 2 b + j -> state j NB + b
+            const int rep = SPILL ? 0 : a.rep_shift;
+            const int i = ((ki & 1) * a.NB + (ki >> 1)) << rep;  // key index 2 b + j -> state j NB + b
             unsigned long long c = 0;
             uint64_t sum = 0;
             __int128 wide = 0;
             long long mn = V32 ? INT_MAX : LLONG_MAX, mx = V32 ? INT_MIN : LLONG_MIN;
 #pragma unroll 1
-            for (int k = 0; k < 1 << a.rep_shift; ++k) {
+            for (int k = 0; k < 1 << rep; ++k) {
                 // lanes start at different copies, so the copies of neighbouring slots are read from different banks
-                const int e = i + ((k + static_cast<int>(threadIdx.x)) & ((1 << a.rep_shift) - 1));
+                const int e = i + ((k + static_cast<int>(threadIdx.x)) & ((1 << rep) - 1));
                 c += cnt[e];
                 if (a.has_sum) {
                     const uint64_t lo = (static_cast<uint64_t>(l1[e]) << 32) | l0[e];
@@ -367,8 +366,8 @@ constexpr int FM_NULL = 32;  // NULL masks (key, value, predicate) or a row mask
 constexpr int FM_WIDE = 64;  // 96-bit sums of floats and doubles
 constexpr int FM_KMOD = 16;  // keys are replaced by key % m as they are read (single INT32 or INT64 key)
 
-// K32: every key word is a 32-bit key's, so none equals kEmpty.  FAR: keys of a full home bucket go to the far one.
-template <typename VT, int MODE, bool K32 = false, bool FAR = false>
+// K32: every key word is a 32-bit key's, so none equals kEmpty.
+template <typename VT, int MODE, bool K32 = false>
 struct FastWarp {
     static constexpr bool SUM = (MODE & FM_SUM) != 0;
     static constexpr bool MM = (MODE & FM_MM) != 0;
@@ -423,7 +422,7 @@ struct FastWarp {
     // Looks kw (hash m, home bucket b, full and without it) up in the next bucket it may be in: the slot or -1.
     __device__ __forceinline__ int look_on(uint64_t kw, uint64_t m, uint32_t b) const {
         bool empty;
-        return fprobe(t, FAR ? ffar(m, t.NB) : fnext(b, t.NB), kw, empty);
+        return fprobe(t, fnext(b, t.NB), kw, empty);
     }
 
     __device__ __forceinline__ void touch_queue(bool put, uint64_t kw, unsigned lane) {
@@ -535,7 +534,7 @@ struct FastWarp {
             for (int u = 0; u < U; ++u) {
                 if (look[u] && !hit[u]) {
                     int s2 = look_on(kw[u], m[u], b[u]);  // a key whose home bucket is full
-                    if (s2 < 0) s2 = fclaim(t, b[u], kw[u], probe_b, FAR);
+                    if (s2 < 0) s2 = fclaim(t, b[u], kw[u], probe_b, false);
                     hit[u] = s2 >= 0;
                     slot[u] = static_cast<uint32_t>(s2);
                 }
@@ -631,7 +630,7 @@ struct FastWarp {
                     go = (atoms_or(seen + (hb >> 5) * 4u, bit) & bit) != 0u;
                 }
                 if (go) {
-                    slot[u] = fclaim(t, b[u], kw[u], fits ? probe_b : 1, FAR);
+                    slot[u] = fclaim(t, b[u], kw[u], fits ? probe_b : 1, !empty[u]);
                     hit[u] = slot[u] >= 0;
                 }
             }
@@ -794,10 +793,11 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
     constexpr bool NUL = !COMP && (MODE & FM_NULL) != 0;
     constexpr bool WIDE = (MODE & FM_WIDE) != 0;
     constexpr bool LIST = HAS_PRED || NUL;  // rows are filtered into the warp's list
-    // Rows a lane takes per step: a warp's whole slice of a tile where every row passes, two where they come off the list
-    // and for sums of doubles, whose four rows do not fit the 96 registers (2^24 rows of int32 keys and double values, SUM
-    // over 3000 groups: 191 us with four, 159 with two).
-    constexpr int U = LIST || (std::is_same<VT, double>::value && (MODE & FM_SUM)) ? 2 : kFastSeg;
+    // Rows a lane takes per step: a warp's whole slice of a tile where every row passes and no values are read, else two:
+    // four rows with values do not fit the 96 registers (2^24 rows over 3000 groups, SUM of double, int32 keys: 191 us with
+    // four, 159 with two; over 30,000 groups, SUM/MIN/MAX/COUNT of int32, int64 keys: 344 and 284.  Tables of wide rows that
+    // hold every group would be 10 to 15 % faster with four, but their code beside the other costs both its registers).
+    constexpr int U = LIST || VALS ? 2 : kFastSeg;
     using PL = typename std::conditional<HAS_PRED, PT, int32_t>::type;
     constexpr int PW = sizeof(PL);
 
@@ -1008,7 +1008,7 @@ __global__ void __launch_bounds__(kFastThreads, 1) gb_fast_kernel(const AggArgs 
             if constexpr (VALS) v = rv[g];
             else v = VT{};
         };
-        // Steps over list entries [e0, e1): full 64-row steps, and the remainder when `flush`.  Returns the entries taken.
+        // Steps over list entries [e0, e1): full steps, and the remainder when `flush`.  Returns the entries taken.
         const bool listed = LIST && (HAS_PRED || a.ptype || a.mask || a.pnull);  // FM_NULL without a filter: every row passes
         auto steps = [&](int total, bool flush, int g0) -> int {
             int e0 = 0;
@@ -1311,7 +1311,7 @@ __global__ void __launch_bounds__(kFSpillThreads<MODE>, 1) gb_fspill_kernel(cons
         __syncthreads();
         const int hb = max(1, 64 - __clzll(static_cast<long long>(total)));
         const FixQ fq = fixq<VT, WIDE>(s_emax == INT_MIN ? 0 : s_emax, hb);
-        FastWarp<VT, MODE, false, true> fw(a, tab, fq, &s_claims);
+        FastWarp<VT, MODE> fw(a, tab, fq, &s_claims);
         fw.bshift = 32 - a.spill_bits;
         fw.fits = a.fits != 0;
         fw.probe_b = a.probe_b;
@@ -1339,7 +1339,7 @@ __global__ void __launch_bounds__(kFSpillThreads<MODE>, 1) gb_fspill_kernel(cons
         __syncthreads();
         for (int i = threadIdx.x; i < parts2; i += blockDim.x)
             a.spill2_fill[static_cast<int64_t>(p) * parts2 + i] = min(fill2[i], static_cast<unsigned>(a.spill2_cell));
-        ftab_flush<VT, WIDE>(sm, a, fq, &s_claims);
+        ftab_flush<VT, WIDE, true>(sm, a, fq, &s_claims);
         __syncthreads();
     }
     if (threadIdx.x == 0) publish_claims(a.counters, a.capacity, s_claims);
