@@ -697,6 +697,24 @@ int32_t qdb_gb_reset(qdb_gb* gb, void* stream) {
     return QDB_OK;
 }
 
+// Whether a masked call is faster in the fast pass than in the general one, whose shared table has `slots` slots.
+//  * Groups that the general pass's table about holds: the fast pass's larger tables cost more to merge and pay off from
+//    2^20 rows, and from 1024 rows a group (2M rows over 3000 groups, NULL values, SUM of double: 133 us here, 97 there;
+//    16M: 301 and 394).  Rows of 8 bytes under a row mask alone are always the general pass's (16M rows over 4 groups, SUM
+//    of int32: 139 and 121 us).
+//  * More groups: the general pass sends misses to the global table; here they are spilled, which pays off from 2^18 rows
+//    (1M rows over 30,000 groups, NULL values, SUM of int64: 161 and 297 us) unless most rows start a group (4M rows over
+//    2M groups, row mask, SUM/MIN/MAX/COUNT of double: 1.4 times as long here).  NULL keys, all of one group, stay on chip
+//    here (16M rows over 8M groups: 0.2 of the general pass's time; 4M rows over 2M groups: 0.4 to 1.5 of it).
+static bool masked_fast(const AggArgs& a, int64_t groups, int slots, int row_bytes) {
+    const int64_t n = a.n;
+    if (groups <= slots + slots / 4) {
+        if (!a.knull0 && !a.vnull && !a.pnull && row_bytes <= 8) return false;
+        return n >= std::max<int64_t>(int64_t(1) << 20, 1024 * groups);
+    }
+    return n >= (int64_t(1) << 18) && (groups <= n / 8 || (a.knull0 && n >= (int64_t(1) << 23)));
+}
+
 // A compressed-key call (kz) or a fused key % m call (km) that the fast pass cannot take: the caller decompresses the
 // keys, or materialises the remainder column, instead.
 constexpr int32_t kNotFused = -1;
@@ -771,19 +789,22 @@ static int32_t process_impl(qdb_gb* gb, const void* const* key_cols, const uint6
     const bool nulls = a.knull0 || a.knull1 || a.vnull || a.pnull;
     // The fast pass takes calls of whole tiles and aligned columns.  NULL masks and a row mask are staged beside the
     // columns in instantiations of their own (a single key column: a composite key with a NULL component lives in
-    // the table's second region, which only the general pass fills).
+    // the table's second region, which only the general pass fills), for calls that masked_fast picks below.
+    // (QDB_AGG_FAST: 0 never, 2 all masked calls that it can take.)
     const bool masked = nulls || mask;
-    if (gb->placement != QDB_PLACE_GLOBAL && n >= kFastT && env_int("QDB_AGG_FAST", 1) != 0 &&
-        (!masked || (!kz && !km && gb->n_key_cols == 1)) &&
+    const int64_t fast = env_int("QDB_AGG_FAST", 1);
+    const bool can_fast =
+        gb->placement != QDB_PLACE_GLOBAL && n >= kFastT && fast != 0 && (!masked || (!kz && !km && gb->n_key_cols == 1)) &&
         (kz || aligned16(a.key0)) && (!a.key1 || aligned16(a.key1)) && (!a.vals || aligned16(a.vals)) &&
-        (!a.pcol || aligned16(a.pcol)) && aligned16(a.knull0) && aligned16(a.vnull) && aligned16(a.pnull) && aligned16(mask)) {
-        bool used = false;
-        a.nul = masked ? 1 : 0;
+        (!a.pcol || aligned16(a.pcol)) && aligned16(a.knull0) && aligned16(a.vnull) && aligned16(a.pnull) && aligned16(mask);
+    bool used = false;
+    if (can_fast && !masked) {
         const int32_t rc = process_fast(gb, a, pred, ptype, s, &used);
         if (rc != QDB_OK || used) return rc;
-        a.nul = 0;
     }
     if (kz || km) return kNotFused;
+    AggArgs af = a;  // of the fast pass, should it take this masked call
+    af.nul = 1;
 
     // Tile and stage plan: stages of about 32 KB (a stage costs a fixed hand-off between the producer and
     // the consumers, so small stages cannot reach the HBM bandwidth), three of them in the ring.
@@ -895,6 +916,10 @@ static int32_t process_impl(qdb_gb* gb, const void* const* key_cols, const uint6
         } else {
             spill_bits = -1;
         }
+    }
+    if (can_fast && masked && (fast == 2 || masked_fast(af, gb->capacity, a.S, ks + (a.vals ? type_size(gb->val_type) : 0)))) {
+        const int32_t rc = process_fast(gb, af, pred, ptype, s, &used);
+        if (rc != QDB_OK || used) return rc;
     }
     SpillArea* spill = nullptr;
     if (spill_bits >= 0) {

@@ -12,6 +12,12 @@ from test_gpu_parity import ALL, _dev, run_both
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def _fast_pass(monkeypatch):
+    """The fast pass takes every masked call that it can, also those that the general one is picked for."""
+    monkeypatch.setenv("QDB_AGG_FAST", "2")
+
+
 def _keys(rng, n, groups, dt):
     k = rng.integers(0, groups, n)
     if dt in (np.float32, np.float64):
@@ -162,3 +168,32 @@ def test_masked_growing_column_stays_on_chip(cuda, monkeypatch, dt):
             best = min(best, e[0].elapsed_time(e[1]) * 1e3)
         us[fast] = best
     assert us["1"] <= us["0"], us
+
+
+@pytest.mark.parametrize("n,groups,dt,aggs,what", [
+    (100_000, 3000, torch.int32, ["sum", "count"], "values"), (2_000_000, 3000, torch.float64, ["sum"], "values"),
+    (4_000_000, 2_000_000, torch.float64, ["min", "max", "sum", "count"], "rows"),
+    (16_000_000, 4, torch.int32, ["sum"], "rows"), (1_000_000, 30_000, torch.int64, ["sum"], "values"),
+    (16_000_000, 100_000, torch.float64, ["max", "avg"], "keys")])
+def test_masked_calls_take_the_faster_pass(cuda, monkeypatch, n, groups, dt, aggs, what):
+    """Which pass takes a masked call: not slower than either of them (a fifth for the measurement)."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    k = torch.randint(0, groups, (n,), generator=g, device="cuda", dtype=torch.int32)
+    v = (torch.rand(n, generator=g, device="cuda") * 1000).to(dt)
+    nulls = torch.randint(-(1 << 63), (1 << 63) - 1, ((n + 63) // 64,), generator=g, device="cuda")
+    kw = {"values": dict(value_nulls=nulls), "keys": dict(key_nulls=[nulls]),
+          "rows": dict(mask=(torch.rand(n, generator=g, device="cuda") < 0.5).to(torch.int8))}[what]
+    t = GroupByTable(aggs, np.int32, {torch.int32: np.int32, torch.int64: np.int64, torch.float64: np.float64}[dt], groups)
+    us = {}
+    for fast in ("1", "0", "2"):
+        monkeypatch.setenv("QDB_AGG_FAST", fast)
+        us[fast] = float("inf")
+        for _ in range(6):
+            t.reset()
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            t.process([k], v, n, sync=False, **kw)
+            e[1].record()
+            torch.cuda.synchronize()
+            us[fast] = min(us[fast], e[0].elapsed_time(e[1]) * 1e3)
+    assert us["1"] <= 1.2 * min(us.values()) + 3, us
