@@ -106,7 +106,8 @@ __device__ __noinline__ int64_t gbs_claim(GbsRec* r, uint64_t pos, uint64_t* are
 
 // Finds or claims the string at byte offset b (n bytes) of the buffer W; returns its slot, or -1 (table or arena
 // full, key too long, or a wait that gave up: the status word says which).  A key of at most 24 bytes lives in its
-// record: its three words (zero-padded) are hashed and compared without loops, the record read as two 16-byte loads.
+// record: its three words (zero-padded) are hashed and compared without loops, in the home slot's record first and then
+// slot by slot, header before record.
 __device__ int64_t gbs_find(const GbsDict& t, const uint64_t* __restrict__ W, int64_t b, int64_t n, unsigned* claims) {
     if (n > kGbsMaxLen) {
         atomicExch(reinterpret_cast<int*>(&t.counters[1]), static_cast<int>(QDB_ERR_TOO_LARGE));
@@ -144,11 +145,16 @@ __device__ int64_t gbs_find(const GbsDict& t, const uint64_t* __restrict__ W, in
     if (shortk) {
         // Most rows find their key's record in its home slot: comparing the key itself there spares them the header, a
         // dependent load of the chain that this pass is bound by.  Anything else takes the full probe below.
-        // One 32-byte load, so meta and words are of one time; meta 0 (unpublished) or poison never matches a length.
+        // The record may be read while it is published, its four words in any order.  Each goes from 0 to its value once,
+        // so an equal word that is not 0 is the published one, and meta 0 (unpublished) or poison never matches a length.
+        // A key with an all-zero word of its own could match a word not yet written: it takes the full probe.
+        bool solid = true;
+#pragma unroll
+        for (int j = 0; j < kGbsInline; ++j) solid = solid & (8 * j >= n || w[j] != 0ull);
         uint64_t m, r0, r1, r2;
         asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
                      : "=l"(m), "=l"(r0), "=l"(r1), "=l"(r2) : "l"(t.rec + pos) : "memory");
-        if (m != kMetaPoison && gbs_meta_len(m) == n && ((r0 == w[0]) & (r1 == w[1]) & (r2 == w[2])))
+        if (solid && m != kMetaPoison && gbs_meta_len(m) == n && ((r0 == w[0]) & (r1 == w[1]) & (r2 == w[2])))
             return static_cast<int64_t>(pos);
     }
     for (uint64_t probe = 0; probe < t.cap; ++probe, pos = (pos + 1) & mask) {
