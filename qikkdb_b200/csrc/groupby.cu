@@ -224,11 +224,6 @@ static void spill_release(SpillArea* A, cudaStream_t s) {
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-static int64_t env_int(const char* name, int64_t dflt) {
-    const char* v = getenv(name);
-    return (v && *v) ? strtoll(v, nullptr, 10) : dflt;
-}
-
 // ---------------------------------------------------------------------------------------------
 // Predicate `col OP constant` -> interval of the column type.  The comparison the reference's
 // kernel_filter makes (OP{}(a, b) on typed operands, in the C++ common type, GPUFilterConditions.cuh:9-120)

@@ -338,15 +338,16 @@ struct ObArgs {
     const uint32_t* start = nullptr; // [digits][256]
     ObPass* pass = nullptr;
     uint64_t* state = nullptr;       // [tiles][256]
+    uint32_t max_polls = 0;          // unsuccessful looks at its predecessors after which a tile helps itself
 };
 
-constexpr uint32_t kObMaxPolls = 1u << 20;
+constexpr int64_t kObMaxPolls = 1 << 20;
 constexpr int kObLook = 8;
 
 // One pass of one tile.  state[t * 256 + d]: high word 2 p + 1 when the low word is the count of digit d in tile t, 2 p
 // + 2 when it is the count in tiles 0..t (p the pass; the words of earlier passes are smaller, so the area is cleared
 // once per column).  Tiles are numbered by a ticket, so a tile's predecessors are running or done; a tile that has
-// polled kObMaxPolls times counts its predecessors' rows itself instead of waiting on.
+// polled a.max_polls times counts its predecessors' rows itself instead of waiting on.
 //
 // Rows leave through shared memory in digit order, so a digit's 16 rows of a tile on average (24 for 32-bit keys) go out
 // in one piece, in two to four store pieces; their number bounds the pass (a row's 24 bytes read and written per digit
@@ -479,7 +480,7 @@ __global__ void __launch_bounds__(kObThreads, 2) ob_pass_kernel(const ObArgs<K> 
                 }
             }
             t -= took;
-            if (took == 0 && ++polls > kObMaxPolls) gave_up = true;
+            if (took == 0 && ++polls > a.max_polls) gave_up = true;
         }
         if (!gave_up) ob_st(my_state, f_inc | (before + count));
     }
@@ -563,6 +564,7 @@ static int32_t ob_column(const void* col, const uint64_t* nulls, int32_t desc, i
     a.out = indices;
     a.n = n;
     a.first = first ? 1 : 0;
+    a.max_polls = static_cast<uint32_t>(env_int("QDB_OB_POLLS", kObMaxPolls));
     constexpr size_t smem = static_cast<size_t>(kObTile<K>) * (sizeof(K) + 4) + kObWarps * 256 * 6;
     cudaError_t e = cudaMemsetAsync(mem, 0, hist_b + pass_b + state_b, s);
     if (e == cudaSuccess) {

@@ -4,6 +4,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <type_traits>
 #include <string>
@@ -51,6 +52,12 @@ void dev_free(void* p, cudaStream_t s);
 // Copies `bytes` (at most 64) from the device on stream s and waits for them, through page-locked memory of the calling
 // thread (a copy into pageable memory goes through a staging buffer of the driver: about 4 us more).
 cudaError_t read_back(void* dst, const void* src, size_t bytes, cudaStream_t s);
+
+// A plan knob from the environment, read on every call.
+inline int64_t env_int(const char* name, int64_t dflt) {
+    const char* v = getenv(name);
+    return (v && *v) ? strtoll(v, nullptr, 10) : dflt;
+}
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 

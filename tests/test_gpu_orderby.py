@@ -147,3 +147,18 @@ def test_order_by_column_of_chosen_rows(cuda, n):
     capi.check(capi.lib().qdb_order_by_column(capi.QDB_INT32, dc.data_ptr(), None, 0, n, 0, idx.data_ptr(),
                                               torch.cuda.current_stream().cuda_stream))
     assert (idx.cpu().numpy() == rows[np.argsort(col[rows], kind="stable")]).all()
+
+
+@pytest.mark.parametrize("polls", [0, 3])
+@pytest.mark.parametrize("dt", [np.int32, np.int64, np.float64])
+def test_order_by_tiles_that_stop_waiting(cuda, monkeypatch, polls, dt):
+    """A tile that has looked for its predecessors' counts in vain `polls` times counts their rows itself: with a limit of
+    0 most tiles do, and the tiles behind them use what those publish."""
+    monkeypatch.setenv("QDB_OB_POLLS", str(polls))
+    n = 300_007
+    rng = np.random.default_rng(polls)
+    cols = [rng.integers(-1000, 1000, n).astype(np.int32), (rng.standard_normal(n) * 1e6).astype(dt)]
+    exp = oracle.order_by(cols, [True, False], [None, None])
+    dev = [_dev(c) for c in cols]
+    for _ in range(5):
+        assert (order_by(dev, [True, False], [None, None]).cpu().numpy() == exp).all()
