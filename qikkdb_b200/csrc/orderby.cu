@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(kObSmallThreads) ob_small_kernel(const ObSmall
 struct ObPass {              // written by ob_meta_kernel, per digit
     uint32_t run;            // 0: every row has the same digit
     uint32_t ordinal;        // passes that run before this one
-    uint32_t last;           // no later pass runs
+    uint32_t left;           // passes that run from this one on (1: it is the last)
     uint32_t ticket;         // next tile
 };
 
@@ -301,19 +301,14 @@ __global__ void __launch_bounds__(256) ob_meta_kernel(uint32_t* __restrict__ his
     __syncthreads();
     if (threadIdx.x == 0) {
         uint32_t o = 0;
-        int last = -1;
         for (int d = 0; d < D; ++d) {
             pass[d].run = trivial[d] ? 0u : 1u;
             pass[d].ordinal = o;
-            pass[d].last = 0u;
             pass[d].ticket = 0u;
-            if (!trivial[d]) {
-                ++o;
-                last = d;
-            }
+            if (!trivial[d]) ++o;
         }
-        if (last >= 0) pass[last].last = 1u;
-        else pass[D - 1].ordinal = 0xffffffffu;  // no pass runs: the last kernel writes the identity
+        for (int d = 0; d < D; ++d) pass[d].left = o - pass[d].ordinal;
+        if (o == 0) pass[D - 1].ordinal = 0xffffffffu;  // no pass runs: the last kernel writes the identity
     }
 }
 
@@ -330,8 +325,7 @@ template <typename K>
 struct ObArgs {
     K* keys0 = nullptr;
     K* keys1 = nullptr;
-    int32_t* idx0 = nullptr;
-    int32_t* idx1 = nullptr;
+    int32_t* idx = nullptr;          // row numbers, in turn with out so that the last pass writes out
     int32_t* out = nullptr;          // the permutation
     int64_t n = 0;
     int32_t first = 0;               // the permutation before the column's first pass is the identity
@@ -381,8 +375,8 @@ __global__ void __launch_bounds__(kObThreads, 2) ob_pass_kernel(const ObArgs<K> 
     const K* __restrict__ keys_in = odd ? a.keys1 : a.keys0;
     K* __restrict__ keys_out = odd ? a.keys0 : a.keys1;
     const bool ident = a.first && ps.ordinal == 0;
-    const int32_t* __restrict__ idx_in = odd ? a.idx1 : a.idx0;
-    int32_t* __restrict__ idx_out = ps.last ? a.out : (odd ? a.idx0 : a.idx1);
+    const int32_t* __restrict__ idx_in = (ps.left & 1u) ? a.idx : a.out;
+    int32_t* __restrict__ idx_out = (ps.left & 1u) ? a.out : a.idx;
     if (threadIdx.x == 0) s_tile = atomicAdd(&a.pass[p].ticket, 1u);
     for (int i = threadIdx.x; i < kObWarps * 256; i += kObThreads) {
         words[i] = 0u;
@@ -501,7 +495,7 @@ __global__ void __launch_bounds__(kObThreads, 2) ob_pass_kernel(const ObArgs<K> 
     for (int i = threadIdx.x; i < rows; i += kObThreads) {
         const K k = s_keys[i];
         const uint32_t g = s_glob[static_cast<uint32_t>(k >> shift) & 0xffu] + static_cast<uint32_t>(i);
-        if (!ps.last) keys_out[g] = k;
+        if (ps.left > 1u) keys_out[g] = k;
         idx_out[g] = s_idx[i];
     }
 }
@@ -545,11 +539,11 @@ static int32_t ob_column(const void* col, const uint64_t* nulls, int32_t desc, i
     static std::atomic<uint64_t> allowed{0};
     int32_t rc = allow_dynamic_smem(reinterpret_cast<const void*>(ob_pass_kernel<K>), allowed, "ob_pass_kernel shared memory");
     if (rc != QDB_OK) return rc;
-    // One allocation: the digit counts, the passes and the tile states (cleared), two key and two row buffers.
+    // One allocation: the digit counts, the passes and the tile states (cleared), two key buffers and one of row numbers.
     const size_t hist_b = D * 256 * sizeof(uint32_t), pass_b = 256, state_b = static_cast<size_t>(tiles) * 256 * 8;
     const size_t key_b = (static_cast<size_t>(n) * sizeof(K) + 255) / 256 * 256, idx_b = (static_cast<size_t>(n) * 4 + 255) / 256 * 256;
     unsigned char* mem = nullptr;
-    rc = dev_alloc(reinterpret_cast<void**>(&mem), hist_b + pass_b + state_b + 2 * key_b + 2 * idx_b, s);
+    rc = dev_alloc(reinterpret_cast<void**>(&mem), hist_b + pass_b + state_b + 2 * key_b + idx_b, s);
     if (rc != QDB_OK) return rc;
     ObArgs<K> a;
     uint32_t* hist = reinterpret_cast<uint32_t*>(mem);
@@ -559,8 +553,7 @@ static int32_t ob_column(const void* col, const uint64_t* nulls, int32_t desc, i
     unsigned char* q = mem + hist_b + pass_b + state_b;
     a.keys0 = reinterpret_cast<K*>(q);
     a.keys1 = reinterpret_cast<K*>(q + key_b);
-    a.idx0 = reinterpret_cast<int32_t*>(q + 2 * key_b);
-    a.idx1 = reinterpret_cast<int32_t*>(q + 2 * key_b + idx_b);
+    a.idx = reinterpret_cast<int32_t*>(q + 2 * key_b);
     a.out = indices;
     a.n = n;
     a.first = first ? 1 : 0;
@@ -571,7 +564,7 @@ static int32_t ob_column(const void* col, const uint64_t* nulls, int32_t desc, i
         const DeviceInfo& di = device_info();
         const unsigned g = static_cast<unsigned>(std::min<int64_t>((n + kObThreads - 1) / kObThreads, int64_t(di.sm_count) * 4));
         ob_keys_kernel<T, K><<<g, kObThreads, 0, s>>>(static_cast<const T*>(col), nulls, first ? nullptr : indices, n, desc,
-                                                      a.keys0, a.idx0, hist);
+                                                      a.keys0, a.idx, hist);
         ob_meta_kernel<D><<<1, 256, 0, s>>>(hist, static_cast<uint32_t>(n), a.pass);
         for (int p = 0; p < D; ++p) ob_pass_kernel<K><<<static_cast<unsigned>(tiles), kObThreads, smem, s>>>(a, p);
         note_launch(2 + D);

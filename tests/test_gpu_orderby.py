@@ -162,3 +162,25 @@ def test_order_by_tiles_that_stop_waiting(cuda, monkeypatch, polls, dt):
     dev = [_dev(c) for c in cols]
     for _ in range(5):
         assert (order_by(dev, [True, False], [None, None]).cpu().numpy() == exp).all()
+
+
+@pytest.mark.parametrize("dt,most", [(np.int32, 13), (np.int64, 21)])
+def test_order_by_scratch(cuda, dt, most):
+    """Scratch of the tiled form: two key buffers, one of row numbers and half a byte of tile states a row."""
+    from cuda.bindings import runtime as rt
+    n = 3_000_000
+    col = torch.from_numpy(np.random.default_rng(1).integers(-1 << 30, 1 << 30, n).astype(dt)).cuda()
+    order_by([col], [False], [None])
+    torch.cuda.synchronize()
+    err, pool = rt.cudaDeviceGetDefaultMemPool(0)
+    assert err == rt.cudaError_t.cudaSuccess
+    attr = rt.cudaMemPoolAttr
+    err, used = rt.cudaMemPoolGetAttribute(pool, attr.cudaMemPoolAttrUsedMemCurrent)
+    assert err == rt.cudaError_t.cudaSuccess
+    (err,) = rt.cudaMemPoolSetAttribute(pool, attr.cudaMemPoolAttrUsedMemHigh, type(used)(0))
+    assert err == rt.cudaError_t.cudaSuccess
+    idx = order_by([col], [False], [None])
+    torch.cuda.synchronize()
+    err, high = rt.cudaMemPoolGetAttribute(pool, attr.cudaMemPoolAttrUsedMemHigh)
+    assert (torch.diff(col[idx.long()]) >= 0).all()
+    assert 0 < int(high) - int(used) <= most * n
