@@ -544,6 +544,8 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
         const int64_t cells2 = spill_bits2 ? (parts << spill_bits2) : 0;
         int32_t rc = spill_acquire(gb->device, spill_bits2 ? 2 * words : words, 0,
                                    parts * ctas + 1 + (spill_bits2 ? cells2 + 1 : 0), s, &spill);
+        // A masked call has the general pass to fall back on, whose area is half as large.
+        if (rc == QDB_ERR_NOMEM && a.nul) return QDB_OK;
         if (rc != QDB_OK) return rc;
         a.spill_keys = spill->keys;
         a.spill_vals = nullptr;

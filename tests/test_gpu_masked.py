@@ -1,10 +1,14 @@
 """The fast aggregation pass over NULL masks and row masks (single keys), against the oracle: every key and value type
 at the edges of its 2048-row tile, tables that hold every group and tables that spill, keys that share the NULL key's
 or the empty slot's word, groups without a non-NULL value, and the accuracy of SUM and AVG of doubles."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
 
+from conftest import ROOT
 from gpu_compare import FLOAT_RTOL
 from qikkdb_b200.groupby import FilterConditions, GroupByTable, device_nullmask
 from test_gpu_parity import ALL, _dev, run_both
@@ -197,3 +201,34 @@ def test_masked_calls_take_the_faster_pass(cuda, monkeypatch, n, groups, dt, agg
             torch.cuda.synchronize()
             us[fast] = min(us[fast], e[0].elapsed_time(e[1]) * 1e3)
     assert us["1"] <= 1.2 * min(us.values()) + 3, us
+
+
+_TIGHT = """
+import numpy as np, os, torch
+from qikkdb_b200.groupby import GroupByTable
+n, groups = 1 << 26, 100_000
+g = torch.Generator(device="cuda").manual_seed(1)
+k = torch.randint(0, groups, (n,), generator=g, device="cuda", dtype=torch.int32)
+v = torch.randint(-1000, 1000, (n,), generator=g, device="cuda")
+mask = (torch.rand(n, generator=g, device="cuda") < 0.5).to(torch.int8)
+t = GroupByTable(["sum", "count"], np.int32, np.int64, groups)
+exp = torch.zeros(groups, dtype=torch.int64, device="cuda").index_add_(0, k.long(), v * mask)
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+free, _ = torch.cuda.mem_get_info()
+hog = torch.empty(free - (1 << 30), dtype=torch.uint8, device="cuda")  # leaves 1 GiB
+t.process([k], v, n, mask=mask)
+del hog
+torch.cuda.empty_cache()
+r = t.results_numpy()
+o = np.argsort(r["keys"][0])
+assert (r["sum"][o] == exp.cpu().numpy()).all()
+print("tight ok")
+"""
+
+
+def test_masked_call_with_little_memory(cuda):
+    """A masked call of 2^26 rows that spills, with 1 GiB of memory left: the fast pass's spill area takes 1.3 GB, the general
+    pass's 0.7, and the call is served as before."""
+    res = subprocess.run([sys.executable, "-c", _TIGHT], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0 and "tight ok" in res.stdout, res.stdout + res.stderr
