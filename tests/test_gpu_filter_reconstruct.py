@@ -106,3 +106,20 @@ def test_prefix_sum_and_compress(cuda):
     arr = (rng.random(n) < 0.5).astype(np.uint8)
     words = GPUReconstruct.CompressNullMask(_dev(arr), n).numpy()
     assert (unpack_nullmask(words, n) == arr.astype(bool)).all()
+
+
+@pytest.mark.parametrize("n", [8192 * 4096, 8192 * 4096 + 1, 2 * 8192 * 4096 + 4097])
+def test_compaction_of_more_tiles_than_one_scan_step(cuda, n):
+    """The scan of the tile counts takes 8192 tiles of 4096 rows a step and carries their total on: columns of one such
+    step, one row more, and three steps, against torch."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    mask = (torch.rand(n, generator=g, device="cuda") < 0.01).to(torch.int8)
+    mask[-1] = 1
+    rows = mask.nonzero().view(-1)
+    for dt in (torch.int8, torch.int32):
+        col = torch.randint(-100, 100, (n,), generator=g, device="cuda", dtype=dt)
+        out, cnt, _ = GPUReconstruct.reconstructColKeep(col, mask, n)
+        assert cnt == rows.numel() and (out.torch() == col[rows]).all()
+    idx, cnt = GPUReconstruct.GenerateIndexesKeep(mask, n)
+    assert cnt == rows.numel() and (idx.torch() == rows).all()
+    assert (GPUReconstruct.PrefixSum(mask, n) == torch.cumsum(mask, 0, dtype=torch.int32)).all()
