@@ -17,7 +17,7 @@ constexpr int kBMaxRowsPerLane = 4;
 constexpr int kBListRows = 256;                     // rows of a stage tile one consumer warp compacts (u16 list)
 constexpr int kBSmemCap = 192 * 1024;              // shared memory per CTA: the rest stays L1 for the probe loads
 // Result extraction: a query's slots in chunks, kBResBlocks blocks per query.  (One block of 1024 threads per query left
-// the largest of a batch's tables to one SM: 552 us for 48 queries of 4 to 16,384 groups.)
+// the largest of a batch's tables to one SM: 552 us for 48 queries of 4 to 65,536 groups.)
 constexpr int kBResThreads = 256;
 constexpr int kBResPer = 4;
 constexpr int kBResChunk = kBResThreads * kBResPer;

@@ -343,9 +343,9 @@ PredInterval pred_interval(const qdb_pred& p) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Plan and launch of the fast pass (groupby_fast.cuh) for a call without NULL masks or a precomputed mask whose
-// columns are 16-byte aligned and hold at least one whole tile.  *used is false when the plan does not fit shared
-// memory (the caller then takes the general pass).
+// Plan and launch of the fast pass (groupby_fast.cuh; groupby_few.cuh for the calls that it names) over columns that are
+// 16-byte aligned and hold at least one whole tile; a.nul: with NULL masks or a row mask.  *used is false when the plan
+// does not fit shared memory, or a masked call's spill area the device's (the caller then takes the general pass).
 // ---------------------------------------------------------------------------------------------
 constexpr int64_t kFewRows = 3072;     // rows of one step of a CTA of the pass without a ring (groupby_few.cuh: 768 x 4)
 constexpr size_t kMaxStates = 8192;  // states of a table with copies (clearing and merging them stays a few us)
@@ -354,7 +354,7 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
     *used = false;
     const DeviceInfo& di = device_info();
     const ValKind vk = val_kind(gb->val_type);
-    // A table whose aggregates never read the values (COUNT only, no NULL masks here) streams the keys alone.
+    // A table whose aggregates never read the values (COUNT only) streams the keys alone (and the value NULLs, a.nul).
     if (fast_mode(a) == 0) a.vals = nullptr;
     const int ks = (gb->n_key_cols == 2) ? 4 : type_size(gb->key_type);
     const int vs = a.vals ? type_size(gb->val_type) : 0;
@@ -457,7 +457,7 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
     }
 
     // Spill plan: partitions small enough for the spill pass's table (one CTA per SM, the largest table shared
-    // memory holds after the cell-fill prefix and the second-level counters) at half load.  The aggregation pass
+    // memory holds after the cell-fill prefix and the second-level counters) at 9/16 load.  The aggregation pass
     // writes at most 2^kMaxSpillBits partitions; a table needing more has two levels: the spill pass over the first
     // level aggregates what its table takes and sends the other rows to 2^spill_bits2 sub-partitions per partition,
     // which a third pass aggregates.  (Measured on 2^27 rows over 16.8M groups: one level of 8192 partitions, whose
@@ -486,8 +486,8 @@ static int32_t process_fast(qdb_gb* gb, AggArgs a, const qdb_pred* pred, int32_t
             const uint64_t parts = std::max(min_parts, next_pow2((static_cast<uint64_t>(gb->capacity) + per - 1) / per));
             int bits = 0;
             while ((1ull << bits) < parts) ++bits;
-            // ... and a table sized for its partition's share of the groups at half load (the spill pass clears and
-            // scans every slot of it per item).
+            // ... and a table sized for its partition's share of the groups, at most half full where shared memory
+            // holds it (the spill pass clears and scans every slot of it per item).
             const uint64_t want = std::max<uint64_t>(64, next_pow2((static_cast<uint64_t>(gb->capacity) + parts - 1) / parts));
             if (want < static_cast<uint64_t>(NB2)) NB2 = static_cast<int>(want);
             const int max1 = static_cast<int>(env_int("QDB_SPILL_BITS_MAX", kMaxSpillBits));

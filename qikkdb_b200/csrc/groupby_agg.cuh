@@ -94,11 +94,11 @@ struct AggArgs {
     int64_t spill_cell = 0;          // rows per cell
     int32_t spill_bits = 0;          // log2 of the partition count
     int32_t spill_ctas = 0;          // CTAs of the aggregation pass (its grid)
-    // Bucketed table of the fast pass (groupby_fast.cuh): NB buckets of four slots, one 64-bit tag word per
-    // bucket at so_tags, key words at so_keys; counts, sum limbs and min/max at so_cnt, so_l0, so_l1, so_mn.
+    // Bucketed table of the fast pass (groupby_fast.cuh): NB buckets of two slots, key words at so_keys; counts, sum limbs
+    // and min/max at so_cnt, so_l0, so_l1, so_l2, so_mn, so_mx.
     int32_t NB = 0;
-    int32_t so_tags = 0, so_keys = 0;
-    int32_t fits = 0;      // 1: every group fits the table: a key may overflow into the next probe_b - 1 buckets
+    int32_t so_keys = 0;
+    int32_t fits = 0;      // 1: every group fits the table: a key may overflow into probe_b - 1 other buckets
     int32_t probe_b = 1;   // buckets a claim may visit
     // Calls of the fast pass with NULL masks or a row mask: the predicate's type (0 none), whether a key may be NULL, sums
     // of floats and doubles in 96 bits (a third limb at so_l2), and the warps' queues of keys to look up.
@@ -109,7 +109,6 @@ struct AggArgs {
     int32_t so_touch = 0;
     int32_t so_mx = 0;       // fast pass: maxima (minima at so_mn; each only when the table has the aggregate)
     int32_t rep_shift = 0; // 2^rep_shift copies of every slot's state (tables of few groups)
-    int32_t pred_float = 0;  // the fast pass compares IEEE predicate values as order-preserving integers
     int32_t flush_rounds = 16;  // lock-step probe rounds of a shared table's merge into the global table
     // Second spill level (fast pass, tables with more partitions than one pass writes well): the spill pass over the
     // first level sends the rows its table cannot take to cell p * 2^spill2_bits + q of this area, q the next

@@ -138,7 +138,9 @@ static __device__ __noinline__ int fclaim(const FTab t, uint32_t b, uint64_t kw,
 // 64-bit fixed-point sum addends.  A CTA that may add up to 2^hb - 1 values into one slot keeps every addend below
 // 2^(63 - hb) in magnitude, so the slot's two's-complement sum cannot overflow.  emax is the largest binary exponent
 // (|v| < 2^emax) of the CTA's first tile; values up to 2^(emax + 2) are kept.
-//   float: q = m24 << sh with sh = biased exponent - sh0 in [0, 39 - hb]: exact.
+//   float: q = m24 << sh with sh = biased exponent - sh0 in [0, min(30, 39 - hb)]: exact.  (The bound of 30 lets one widening
+//   multiply shift and sign-extend; it narrows the window of spill items of fewer than 512 rows only, whose values below
+//   2^-28 of the largest are added in FP64.)
 //   double: q = round(v * 2^F) for |v| in [lo, hi): every kept value has at least 24 significant bits.
 // FM_WIDE (calls with NULL masks or a row mask) keeps sums in 96 bits (three limbs), so that 64-bit addends need no
 // headroom and the window is wide enough for columns that grow along their rows: values up to 2^(emax + 15) and down to
@@ -146,7 +148,8 @@ static __device__ __noinline__ int fclaim(const FTab t, uint32_t b, uint64_t kw,
 // took 7.3 ms in FP64 atomics on ten words, 0.11 ms in the general pass.)
 //   float: q = m24 << sh with sh in [0, 38]: exact.
 //   double: q = round(v * 2^F) for |v| < 2^(emax + 2) and round(v * 2^(F - 13)) << 13 above, F = 61 - emax, less for CTAs
-//   of 2^19 rows and more so that 2^hb values of 2^(emax + 15) fit 96 bits: at least 37 bits of any kept value.
+//   of 2^19 rows and more so that 2^hb values of 2^(emax + 15) fit 96 bits: 37 bits of the smallest kept value and more
+//   of the others, 24 in CTAs of 2^32 rows.
 // ---------------------------------------------------------------------------------------------
 struct FixQ {
     int sh0 = 0;

@@ -344,9 +344,11 @@ constexpr int kObLook = 8;
 // polled a.max_polls times counts its predecessors' rows itself instead of waiting on.
 //
 // Rows leave through shared memory in digit order, so a digit's 16 rows of a tile on average (24 for 32-bit keys) go out
-// in one piece, in two to four store pieces; their number bounds the pass (a row's 24 bytes read and written per digit
-// would take 36 us).  10M rows of 64-bit keys: 98 us a digit, where histogram, scan and scatter took 117; of 32-bit
-// keys 67 us.  Tiles of 256 or 1024 threads, 14 keys a thread or other look-back widths: 98 to 106 us.
+// in one piece.  10M rows of 64-bit keys: 98 us a digit, where histogram, scan and scatter took 117; of 32-bit keys 67 us.
+// The 24 bytes read and written per row would take 36 us and the 2.2M pieces of a pass about 55 at 40 G/s; what makes up
+// the rest is not settled.  Tiles of 1024 threads or 14 keys a thread, with half the pieces, tiles of 256 threads and other
+// look-back widths all take 98 to 106 us, so neither the pieces nor the look-back alone bound it; the chain of the rank
+// loop (an atomic, a read and a write per step and warp) and the seven barriers of a tile have not been taken apart.
 template <typename K>
 __global__ void __launch_bounds__(kObThreads, 2) ob_pass_kernel(const ObArgs<K> a, int p) {
     constexpr int ITEMS = kObItems<K>;

@@ -1,6 +1,7 @@
-"""The aggregation pass of tables that hold every group (no ring, no spill), against the oracle: every key and value type
-at the edges of its steps (2 or 4 rows a thread, 768 threads, one CTA per SM), predicates of every type, keys that never
-enter a shared table, values outside the fixed-point window, and tables up to the most groups the pass takes."""
+"""Tables that hold every group, against the oracle: the pass without a ring (4-byte keys and values, no predicate) at the
+edges of its steps (2 or 4 rows a thread, 768 threads, one CTA per SM) and up to the most groups it takes, and the staged
+pass for 8-byte keys and values and predicates of every type; keys that never enter a shared table, values outside the
+fixed-point window; and that each of them is the faster one for its calls."""
 import numpy as np
 import pytest
 import torch

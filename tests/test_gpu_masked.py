@@ -81,9 +81,9 @@ def test_masked_all_rows_null_or_filtered(cuda):
 
 @pytest.mark.parametrize("groups", [50, 40_000])
 def test_masked_double_sums(cuda, groups):
-    """Doubles under NULL masks are summed in 96-bit fixed point: 2^-62 of the largest value per addend.  Partial sums
-    meet in FP64 atomics (at most 148 CTAs' per group), so the relative error of a sum of positive values of like size
-    stays below 148 x 2^-53 + the window's 2^-40 for the smallest values it keeps."""
+    """Doubles under NULL masks are summed in 96-bit fixed point: within 2^-62 of the first tile's largest value per
+    addend, or 2^-49 of it for the few above 2^2 times that.  Partial sums meet in FP64 atomics (at most 148 CTAs' per
+    group), so the relative error of a sum of positive values of like size stays below 148 x 2^-53 + 2^-49."""
     n = 2_000_003
     rng = np.random.default_rng(groups)
     k = rng.integers(0, groups, n)
@@ -171,7 +171,7 @@ def test_masked_growing_column_stays_on_chip(cuda, monkeypatch, dt):
             torch.cuda.synchronize()
             best = min(best, e[0].elapsed_time(e[1]) * 1e3)
         us[fast] = best
-    assert us["1"] <= us["0"], us
+    assert us["1"] <= 1.25 * us["0"], us  # a quarter for the measurement; 67 times as long when rows leave the window
 
 
 @pytest.mark.parametrize("n,groups,dt,aggs,what", [
